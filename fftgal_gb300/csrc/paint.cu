@@ -984,7 +984,12 @@ paint_coop_kernel(PaintParams pp, const uint32_t *__restrict__ off, const uint4 
                         // padding cells take 0 x scale, as the reference scales the
                         // whole padded grid (src/fft.c:127-129): NaN for an empty catalog
                         float v0 = 0.f * sc0, v1 = 0.f * sc1;
-                        if (lane < te2) {
+                        if (lane >= te2) {
+                            // a narrower tile's columns beyond te2 took its stencils'
+                            // outer cells: they are cells of a wider tile to come
+                            a0[lane] = 0u;
+                            if (ngr > 1) a1[lane] = 0u;
+                        } else {
                             const uint32_t c0 = a0[lane];
                             a0[lane] = 0u;
                             v0 = __uint2float_rn(c0) * sc0;
