@@ -23,14 +23,20 @@
 //               accumulates their weights in shared memory and writes every
 //               owned cell exactly once (no global atomics, no zeroing pass).
 //
-// FP32 grids (paint_coop_kernel, persistent over tiles): each lane prepares
-// one particle (cell indices and the 3 x 4 weights of one grid) in shared
-// memory, then the warp deposits the particles one at a time with lane =
-// (grid, i row, j row), each lane adding its 4 k cells; the shared layout makes
-// every such step touch 32 distinct banks.  One grid of 32-row tiles, or two
-// of 16-row tiles, take 79 KB of sums: two 512-thread CTAs per SM.  The two
-// interlacing grids of 32-row tiles are painted by separate CTAs, one grid
-// each, from one sort.  Sums are 32-bit fixed point with a
+// FP32 grids with Ng >= 64 (paint_rot_kernel, persistent over tiles of
+// 32 x 16 x 32 cells, two 512-thread CTAs per SM): one thread deposits one
+// particle, each lane of a warp visiting its particle's 64 cells in an order that
+// puts the warp's 32 atomics of every step in 32 distinct banks.  The two
+// interlacing grids are painted by separate CTAs, one grid each, from one sort.
+// Both grids of 1e8 particles at Ng = 1024: 6.67 ms, against 10.67 ms of a warp
+// that staged 32 particles' weights in shared memory and deposited two
+// particles per step, lane = (particle, i row, j row).
+// Smaller FP32 grids (paint_coop_kernel, 16 x 16 x 32 tiles, one or both grids per
+// CTA, tiles that may span the periodic box) keep that staged deposit: each lane
+// prepares one particle (cell indices and the 3 x 4 weights of one grid) in
+// shared memory, then the warp deposits the particles one (two grids) or two
+// (one grid) at a time, each lane adding its 4 k cells.
+// Sums are 32-bit fixed point with a
 // per-tile scale 2^-s, s the largest value for which no cell can exceed 2^32 (a
 // particle adds at most (2/3)^3 of its weight to a cell): the tile's particle
 // total bounds every cell, and only where that bound leaves fewer than 21
@@ -53,7 +59,7 @@
 namespace fg {
 
 constexpr int kTileExt[3] = {16, 16, 32};    // i, j, k
-constexpr int kTileExt1[3] = {32, 16, 32};   // FP32 paints of one grid (Ng >= 64)
+constexpr int kTileExt1[3] = {32, 16, 32};   // FP32 grids with Ng >= 64
 constexpr int kMaxPaintGrids = 2;
 // dense tiles (fewer 32-bit fraction bits than kWideBelow): 64-bit sums with
 // kWideBits fraction bits, one grid per pass.  At 16-19 bits the 32-bit sums
@@ -79,17 +85,9 @@ constexpr uint32_t kOut = 255u;
 static_assert(15 * kSI + 15 * kSJ + kSJ <= kGS, "tile does not fit the layout");
 static_assert(32 + 2 * kPadK <= kSJ, "row padding");
 static_assert(kSI % 32 == 8 && kSJ % 32 == 6 && kGS % 2 == 1, "bank layout");
-// the accumulators: two grids of 16 i rows, or one grid of 32 i rows (row li
-// at li * kSI)
-constexpr int kAccWords = 2 * kGS > 32 * kSI ? 2 * kGS : 32 * kSI;
-static_assert(31 * kSI + 15 * kSJ + kSJ <= kAccWords, "32-row tile does not fit the layout");
+// two grids of 16 i rows, or a dense tile's 64-bit sums of one
+constexpr int kAccWords = 2 * kGS > 2 * 16 * kSI ? 2 * kGS : 2 * 16 * kSI;
 constexpr size_t kAccBytes = (sizeof(uint32_t) * kAccWords + 15) / 16 * 16;
-// The tile-paint CTA: 512 threads, two CTAs per SM, the two grids of 16 i
-// rows at stride kGS or one grid of 32 rows.  (One 1024-thread CTA per SM
-// holding both grids of 32-row tiles, 158 KB of sums, was measured slower than
-// two one-grid CTAs per SM.)  A dense tile's 64-bit sums hold 16 i rows.
-constexpr int kWideRows = kAccWords / 2 / kSI;
-static_assert(kWideRows == 16, "64-bit rows");
 // largest fixed-point scale: products stay below 2^22 so the FMA trick of
 // deposit4 converts them to integers exactly
 constexpr int kMaxFixBits = 23;
@@ -179,13 +177,14 @@ __device__ __forceinline__ void coord(double x, const AxisParams &a, int g, int 
     b = (g1 % Ng + Ng) % Ng;
 }
 
-__device__ __forceinline__ void pcs_weights(float d, float w[4]) {
-    const float e = 1.f - d;
-    const float d2 = d * d;
-    w[0] = e * e * e * (1.f / 6.f);
-    w[1] = ((3.f * d - 6.f) * d2 + 4.f) * (1.f / 6.f);
-    w[2] = (((-3.f * d + 3.f) * d + 3.f) * d + 1.f) * (1.f / 6.f);
-    w[3] = d2 * d * (1.f / 6.f);
+// (explicit operations: every kernel rounds the weights alike; s = 1/6 times a
+// power of two, which scales the weights exactly)
+__device__ __forceinline__ void pcs_weights(float d, float w[4], float s = 1.f / 6.f) {
+    const float e = __fsub_rn(1.f, d), d2 = __fmul_rn(d, d);
+    w[0] = __fmul_rn(__fmul_rn(__fmul_rn(e, e), e), s);
+    w[1] = __fmul_rn(__fmaf_rn(__fmaf_rn(3.f, d, -6.f), d2, 4.f), s);
+    w[2] = __fmul_rn(__fmaf_rn(__fmaf_rn(__fmaf_rn(-3.f, d, 3.f), d, 3.f), d, 1.f), s);
+    w[3] = __fmul_rn(__fmul_rn(d2, d), s);
 }
 
 __device__ __forceinline__ void pcs_weights(double d, double w[4]) {
@@ -461,6 +460,7 @@ __device__ int tile_segment(const PaintParams &pp, const uint32_t *__restrict__ 
     if (q < ncomb) {
         const int idx[3] = {q / (nopt[1] * nopt[2]), (q / nopt[2]) % nopt[1], q % nopt[2]};
         int ot[3], oc[3];
+        bool own = true;
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
             const int nt = pp.nt[a], x = idx[a];
@@ -468,6 +468,7 @@ __device__ int tile_segment(const PaintParams &pp, const uint32_t *__restrict__ 
                 ot[a] = tt[a];
                 oc[a] = nt == 1 ? 0 : x;
             } else {
+                own = false;
                 const int lo = (tt[a] + nt - 1) % nt, hi = (tt[a] + 1) % nt;
                 if (nt == 2) {
                     ot[a] = hi;
@@ -479,8 +480,13 @@ __device__ int tile_segment(const PaintParams &pp, const uint32_t *__restrict__ 
             }
         }
         const long key = (((long)ot[0] * nt1 + ot[1]) * nt2 + ot[2]) * 27 + oc[0] * 9 + oc[1] * 3 + oc[2];
-        b = off[key];
-        cnt = off[key + 1] - b;
+        if (!own) {
+            b = off[key];
+            cnt = off[key + 1] - b;
+        } else if (q == 0) {  // every class of the own tile: 27 adjacent keys, one segment
+            b = off[key];
+            cnt = off[key + 27] - b;
+        }
     }
     return ncomb;
 }
@@ -545,12 +551,7 @@ __device__ __forceinline__ uint32_t pack_local(int b, int Ng, int t0, int te, ui
 // i row, j row) when one grid is painted; every lane adds its row's 4 k
 // cells.  By the bank layout each of the 4 atomic steps is a single
 // shared-memory wavefront (two grids).  The loop is unrolled so that the
-// shared loads of the next particles overlap the atomics of the current one
-// (unrolled by 4: 2 % faster than by 2 at Ng = 1024).  One grid: 32
-// particles staged per round by all lanes and the half warps depositing
-// alternate ones took the one-grid tile paint from 11.7 to 6.9 ms at Ng=1024
-// (with the grid count a template parameter of the kernel, which also took
-// the two-grid paint from 12.4 to 11.9 ms).
+// shared loads of the next particles overlap the atomics of the current one.
 // Stencil cells outside the tile (local index kOut) are skipped.
 // slot of particle p of grid g in the stage buffer: the two grids' records
 // interleave so that lanes reading both fall in different banks
@@ -613,26 +614,110 @@ __device__ __forceinline__ void deposit_all(uint32_t *acc, const StageBuf &sb, i
     } else {
         // one grid: 32 particles staged in slots 0..31, the half warps
         // deposit alternate ones; unrolled fully, so that the shared loads of
-        // later particles are issued among the atomics of earlier ones (10.65
-        // ms against 10.87 by 8, 11.18 by 4, 11.45 by 2 and 11.97 by 1, both
-        // grids at Ng = 1024)
+        // later particles are issued among the atomics of earlier ones
 #pragma unroll 16
         for (int p = h; p < np; p += 2) deposit_one<WIDE, FAST>(acc, sb, p, 0, a, b, lane_off);
     }
 }
 
-// largest fixed-point exponent s for which `n` contributors to one cell cannot
-// overflow its 32-bit sum: each adds round(w 2^s) <= 8/27 2^s + 1/2 (the
-// largest PCS weight product is (2/3)^3), so n (16 2^s + 27) < 54 2^32 is
-// required.  Exact integer arithmetic; a result below kWideBelow selects the
-// 64-bit sums.
+// largest fixed-point exponent s <= kMaxFixBits for which `n` contributors to
+// one cell cannot overflow its 32-bit sum: each adds round(w 2^s) <= 8/27 2^s +
+// 1/2 (the largest PCS weight product is (2/3)^3), so n (16 2^s + 28) <= 54 2^32
+// suffices; -1 if none.  Exact integer arithmetic; a result below kWideBelow
+// selects the 64-bit sums.
 __device__ __forceinline__ int fix_bits_for(uint32_t n) {
-    if (n == 0) return kMaxFixBits;
-    const unsigned long long x = (54ull << 32) / n;
-    if (x <= 28) return -1;
-    const unsigned long long q = (x - 28) >> 4;
-    const int fb = q == 0 ? -1 : 63 - __clzll((long long)q);
-    return fb > kMaxFixBits ? kMaxFixBits : fb;
+    int s = kMaxFixBits;
+    while (s >= 0 && (unsigned long long)n * ((16u << s) + 28u) > (54ull << 32)) --s;
+    return s;
+}
+
+// Fixed-point exponent of a tile of `total` particles.  The total bounds
+// every cell's contributor count; only when that bound leaves fewer than
+// kBlockCountBelow bits are the particles counted per 4^3 block of grid-0 base
+// cells (over the tile plus a 4-cell margin, or the whole periodic axis when
+// one tile spans it).  index(q) is the sorted index of the tile's q-th
+// particle; blk (kBlkN words) and tmp (kBlkN words) are scratch.  Every thread
+// of the CTA takes part.
+template <typename Index>
+__device__ __forceinline__ int tile_fixbits(uint32_t total, const uint4 *__restrict__ sorted, Index index,
+                                            const PaintParams &pp, const TileSegs &ts, const bool *cyc, uint32_t *blk,
+                                            uint32_t *tmp, uint32_t *scan_ws, int *fixbits_s) {
+    const int fixbits = fix_bits_for(total);
+    if (fixbits >= kBlockCountBelow) return fixbits;
+    const int Ng = pp.Ng, fb = pp.fb, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nwarp = kPaintThreads / 32;
+    int nb[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) nb[a] = cyc[a] ? (Ng + kBlk - 1) / kBlk : blk_dim(a);
+    for (int e = tid; e < kBlkN; e += kPaintThreads) blk[e] = 0u;
+    __syncthreads();
+    for (uint32_t q = tid; q < total; q += kPaintThreads) {
+        const uint4 r = sorted[index(q)];
+        const uint32_t rw[3] = {r.x, r.y, r.z};
+        int bidx = 0;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const int b = (int)(rw[a] >> fb);
+            int bb;
+            if (cyc[a]) {
+                bb = b / kBlk;
+            } else {
+                int l = b - ts.t0[a];
+                if (l > Ng / 2) l -= Ng;
+                if (l < -Ng / 2) l += Ng;
+                bb = (l + 4) / kBlk;  // margin of 4 cells below the tile
+                bb = bb < 0 ? 0 : (bb >= nb[a] ? nb[a] - 1 : bb);
+            }
+            bidx = bidx * blk_dim(a) + bb;
+        }
+        atomicAdd(&blk[bidx], 1u);
+    }
+    __syncthreads();
+    // A cell's contributors have grid-0 base cells from 3 below to 3
+    // above it per axis, within 3 consecutive blocks (cyclically on a
+    // periodic axis): the largest 3x3x3 block sum bounds every cell's
+    // contributor count.  Separable window sums along k, j, i.
+    const int D1 = blk_dim(1), D2 = blk_dim(2);
+    for (int e = tid; e < kBlkN; e += kPaintThreads) {
+        const int k = e % D2, j = (e / D2) % D1, i = e / (D2 * D1);
+        uint32_t v = 0;
+        const bool in = i < nb[0] && j < nb[1] && k < nb[2] && (cyc[2] || k + 2 < nb[2]);
+        if (in)
+            for (int c = 0; c < 3; ++c) v += blk[(i * D1 + j) * D2 + (cyc[2] ? (k + c) % nb[2] : k + c)];
+        tmp[e] = v;
+    }
+    __syncthreads();
+    for (int e = tid; e < kBlkN; e += kPaintThreads) {
+        const int k = e % D2, j = (e / D2) % D1, i = e / (D2 * D1);
+        uint32_t v = 0;
+        const bool in = i < nb[0] && j < nb[1] && k < nb[2] && (cyc[1] || j + 2 < nb[1]);
+        if (in)
+            for (int c = 0; c < 3; ++c) v += tmp[(i * D1 + (cyc[1] ? (j + c) % nb[1] : j + c)) * D2 + k];
+        blk[e] = v;
+    }
+    __syncthreads();
+    uint32_t mx = 0;
+    for (int e = tid; e < kBlkN; e += kPaintThreads) {
+        const int k = e % D2, j = (e / D2) % D1, i = e / (D2 * D1);
+        const bool in = i < nb[0] && j < nb[1] && k < nb[2] && (cyc[0] || i + 2 < nb[0]);
+        if (in) {
+            uint32_t v = 0;
+            for (int c = 0; c < 3; ++c) v += blk[((cyc[0] ? (i + c) % nb[0] : i + c) * D1 + j) * D2 + k];
+            mx = max(mx, v);
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if (lane == 0) scan_ws[warp] = mx;
+    __syncthreads();
+    if (tid == 0) {
+        uint32_t m = 0;
+        for (int w = 0; w < nwarp; ++w) m = max(m, scan_ws[w]);
+        *fixbits_s = fix_bits_for(m);
+    }
+    __syncthreads();
+    const int bits = *fixbits_s;
+    return bits;
 }
 
 // Pass B over the tile's records: each warp stages 16 particles for both
@@ -749,7 +834,7 @@ __device__ __forceinline__ void paint_records(uint32_t *acc, StageBuf &sb, const
 template <int NGR>
 __global__ void __launch_bounds__(kPaintThreads, 2)
 paint_coop_kernel(PaintParams pp, const uint32_t *__restrict__ off, const uint4 *__restrict__ sorted,
-                  PaintOut po, unsigned ntiles, int gsplit) {
+                  PaintOut po, unsigned ntiles) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint32_t *acc = reinterpret_cast<uint32_t *>(smem_raw);                 // [2][kGS]
     StageBuf *stage = reinterpret_cast<StageBuf *>(smem_raw + kAccBytes);  // [warps]
@@ -791,12 +876,7 @@ paint_coop_kernel(PaintParams pp, const uint32_t *__restrict__ off, const uint4 
 
     const int Ng = pp.Ng, ngr = NGR;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = kPaintThreads / 32;  // launched with kPaintThreads
-    // gsplit (NGR = 1 with pp.ngrids = 2): even CTAs paint grid 0 and odd
-    // CTAs grid 1 of the same tiles, from one sort keyed for both grids
-    const int mg = (NGR == 1 && gsplit) ? (int)(blockIdx.x & 1) : 0;  // the grid of a one-grid CTA
-    const unsigned cta = (NGR == 1 && gsplit) ? blockIdx.x >> 1 : blockIdx.x;
-    const unsigned ncta = (NGR == 1 && gsplit) ? gridDim.x >> 1 : gridDim.x;
-    unsigned tile = cta;
+    unsigned tile = blockIdx.x;
     if (tile >= ntiles) return;
     for (int e = tid; e < (int)(kAccBytes / 16); e += kPaintThreads)
         reinterpret_cast<uint4 *>(smem_raw)[e] = make_uint4(0, 0, 0, 0);
@@ -806,7 +886,6 @@ paint_coop_kernel(PaintParams pp, const uint32_t *__restrict__ off, const uint4 
         const int ncomb = tile_segment(pp, off, tile, tid, b, cnt);
         tile_publish(ncomb, b, cnt, seg_begin, seg_pref, scan_ws, ts);  // also orders the clearing above
     }
-    const int fb = pp.fb;
     for (;;) {
         tile_geometry(pp, tile, ts);
         const uint32_t total = ts.total;
@@ -816,92 +895,13 @@ paint_coop_kernel(PaintParams pp, const uint32_t *__restrict__ off, const uint4 
         for (int a = 0; a < 3; ++a) cyc[a] = ts.te[a] == Ng;
         build_tabs(ts.te[0], ts.te[1]);
 
-        // fixed-point scale: the tile's particle total bounds every cell's
-        // contributor count; only when that bound leaves fewer than
-        // kBlockCountBelow bits are the particles counted per 4^3 block of grid-0 base cells (over the tile
-        // plus a 4-cell margin, or the whole periodic axis when one tile spans it)
-        int fixbits = fix_bits_for(total);
-        if (fixbits < kBlockCountBelow) {
-            int nb[3];
-#pragma unroll
-            for (int a = 0; a < 3; ++a) nb[a] = cyc[a] ? (Ng + kBlk - 1) / kBlk : blk_dim(a);
-            for (int e = tid; e < kBlkN; e += kPaintThreads) blk[e] = 0u;
-            __syncthreads();
-            for (uint32_t q = tid; q < total; q += kPaintThreads) {
-                const uint4 r = sorted[seg_index(q, seg_begin, seg_pref, nseg)];
-                const uint32_t rw[3] = {r.x, r.y, r.z};
-                int bidx = 0;
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    const int b = (int)(rw[a] >> fb);
-                    int bb;
-                    if (cyc[a]) {
-                        bb = b / kBlk;
-                    } else {
-                        int l = b - ts.t0[a];
-                        if (l > Ng / 2) l -= Ng;
-                        if (l < -Ng / 2) l += Ng;
-                        bb = (l + 4) / kBlk;  // margin of 4 cells below the tile
-                        bb = bb < 0 ? 0 : (bb >= nb[a] ? nb[a] - 1 : bb);
-                    }
-                    bidx = bidx * blk_dim(a) + bb;
-                }
-                atomicAdd(&blk[bidx], 1u);
-            }
-            __syncthreads();
-            // A cell's contributors have grid-0 base cells from 3 below to 3
-            // above it per axis, within 3 consecutive blocks (cyclically on a
-            // periodic axis): the largest 3x3x3 block sum bounds every cell's
-            // contributor count.  Separable window sums along k, j, i; tmp
-            // reuses the stage area.
-            uint32_t *tmp = reinterpret_cast<uint32_t *>(stage);
-            const int D1 = blk_dim(1), D2 = blk_dim(2);
-            for (int e = tid; e < kBlkN; e += kPaintThreads) {
-                const int k = e % D2, j = (e / D2) % D1, i = e / (D2 * D1);
-                uint32_t v = 0;
-                const bool in = i < nb[0] && j < nb[1] && k < nb[2] && (cyc[2] || k + 2 < nb[2]);
-                if (in)
-                    for (int c = 0; c < 3; ++c) v += blk[(i * D1 + j) * D2 + (cyc[2] ? (k + c) % nb[2] : k + c)];
-                tmp[e] = v;
-            }
-            __syncthreads();
-            for (int e = tid; e < kBlkN; e += kPaintThreads) {
-                const int k = e % D2, j = (e / D2) % D1, i = e / (D2 * D1);
-                uint32_t v = 0;
-                const bool in = i < nb[0] && j < nb[1] && k < nb[2] && (cyc[1] || j + 2 < nb[1]);
-                if (in)
-                    for (int c = 0; c < 3; ++c) v += tmp[(i * D1 + (cyc[1] ? (j + c) % nb[1] : j + c)) * D2 + k];
-                blk[e] = v;
-            }
-            __syncthreads();
-            uint32_t mx = 0;
-            for (int e = tid; e < kBlkN; e += kPaintThreads) {
-                const int k = e % D2, j = (e / D2) % D1, i = e / (D2 * D1);
-                const bool in = i < nb[0] && j < nb[1] && k < nb[2] && (cyc[0] || i + 2 < nb[0]);
-                if (in) {
-                    uint32_t v = 0;
-                    for (int c = 0; c < 3; ++c) v += blk[((cyc[0] ? (i + c) % nb[0] : i + c) * D1 + j) * D2 + k];
-                    mx = max(mx, v);
-                }
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-            if (lane == 0) scan_ws[warp] = mx;
-            __syncthreads();
-            if (tid == 0) {
-                uint32_t m = 0;
-                for (int w = 0; w < nwarp; ++w) m = max(m, scan_ws[w]);
-                fixbits_s = fix_bits_for(m);
-            }
-            __syncthreads();
-            fixbits = fixbits_s;
-        }
-        // a dense tile paints one grid per pass into 64-bit sums (one half of
-        // a 32-row tile at a time: 16 rows of 64-bit sums fill the shared
-        // memory); otherwise one pass paints every grid into 32-bit sums
+        const int fixbits = tile_fixbits(
+            total, sorted, [&](uint32_t q) { return seg_index(q, seg_begin, seg_pref, nseg); }, pp, ts, cyc, blk,
+            reinterpret_cast<uint32_t *>(stage), scan_ws, &fixbits_s);
+        // a dense tile paints one grid per pass into 64-bit sums; otherwise one
+        // pass paints every grid into 32-bit sums
         const bool wide = fixbits < kWideBelow;
-        const int nhalf = (wide && ts.te[0] > kWideRows) ? 2 : 1;
-        const int npass = wide ? ngr * nhalf : 1;
+        const int npass = wide ? ngr : 1;
         const float fscale = ldexpf(1.0f, wide ? kWideBits : fixbits);
         if (wide) {
             // the 32-bit tiles leave sums in the row padding: clear all of it
@@ -911,24 +911,17 @@ paint_coop_kernel(PaintParams pp, const uint32_t *__restrict__ off, const uint4 
             __syncthreads();
         }
         const bool fast = !(cyc[0] || cyc[1] || cyc[2]);
-        const unsigned next = tile + ncta;
+        const unsigned next = tile + gridDim.x;
         uint32_t nb_begin = 0, nb_cnt = 0;
         int nb_comb = 0;
         for (int pass = 0; pass < npass; ++pass) {
-            const int pg = NGR == 1 ? mg : pass / nhalf;  // the grid of a wide pass
-            TileSegs tv = ts;             // and its rows
-            if (nhalf == 2) {
-                const int ph = pass % nhalf;
-                tv.t0[0] = ts.t0[0] + kWideRows * ph;
-                tv.te[0] = ph ? ts.te[0] - kWideRows : kWideRows;
-                build_tabs(tv.te[0], tv.te[1]);
-            }
+            const int pg = pass;  // the grid of a wide pass
             if (wide)
-                paint_records<1, true>(acc, stage[warp], sorted, seg_begin, seg_pref, tv, pp, cyc, fast, fscale, pg,
+                paint_records<1, true>(acc, stage[warp], sorted, seg_begin, seg_pref, ts, pp, cyc, fast, fscale, pg,
                                        loctab, masktab, lane, warp);
             else
-                paint_records<NGR, false>(acc, stage[warp], sorted, seg_begin, seg_pref, ts, pp, cyc, fast, fscale,
-                                                   mg, loctab, masktab, lane, warp);
+                paint_records<NGR, false>(acc, stage[warp], sorted, seg_begin, seg_pref, ts, pp, cyc, fast, fscale, 0,
+                                          loctab, masktab, lane, warp);
             __syncthreads();
 
             // the next tile's segments, loaded now and published after the write-out
@@ -951,9 +944,8 @@ paint_coop_kernel(PaintParams pp, const uint32_t *__restrict__ off, const uint4 
                     const float scf = (float)scd;
                     const int accu = po.accumulate[pg];
                     const unsigned long long *acc64 = reinterpret_cast<const unsigned long long *>(acc);
-                    const long vbase = ((long)tv.t0[0] * Ng + tv.t0[1]) * rstride + tv.t0[2];
-                    for (int li = warp; li < tv.te[0]; li += nwarp) {
-                        float *o = reinterpret_cast<float *>(po.out[pg]) + vbase + li * istride;
+                    for (int li = warp; li < ts.te[0]; li += nwarp) {
+                        float *o = reinterpret_cast<float *>(po.out[pg]) + obase + li * istride;
                         const unsigned long long *a = acc64 + kPadK + li * kSI;
                         for (int lj = 0; lj < te1; ++lj, o += rstride, a += kSJ) {
                             float v = 0.f * scf;
@@ -971,12 +963,11 @@ paint_coop_kernel(PaintParams pp, const uint32_t *__restrict__ off, const uint4 
                     __syncthreads();
                     continue;
                 }
-                // grid 0 here is the CTA's grid mg when it paints one grid
-                const float sc0 = (float)ldexp(mg ? s1 : s0, -fixbits);
+                const float sc0 = (float)ldexp(s0, -fixbits);
                 const float sc1 = ngr > 1 ? (float)ldexp(s1, -fixbits) : 0.f;
-                const int accu0 = po.accumulate[mg];
+                const int accu0 = po.accumulate[0];
                 for (int li = warp; li < ts.te[0]; li += nwarp) {
-                    float *o0 = reinterpret_cast<float *>(po.out[mg]) + obase + li * istride;
+                    float *o0 = reinterpret_cast<float *>(po.out[0]) + obase + li * istride;
                     float *o1 = ngr > 1 ? reinterpret_cast<float *>(po.out[1]) + obase + li * istride : nullptr;
                     uint32_t *a0 = acc + kPadK + li * kSI;
                     uint32_t *a1 = a0 + kGS;
@@ -1019,6 +1010,479 @@ paint_coop_kernel(PaintParams pp, const uint32_t *__restrict__ off, const uint4 
         // the clearing above completes before the next deposit: tile_publish
         // synchronises the CTA
         tile_publish(nb_comb, nb_begin, nb_cnt, seg_begin, seg_pref, scan_ws, ts);
+        tile = next;
+    }
+}
+
+// ---- 4b. tile paint of FP32 grids with Ng >= 64: one thread per particle ------------------
+// A tile holds one grid's sums of 32 x 16 x 32 cells in blocks of 2 x 4 x 4
+// cells: cell (i, j, k') of a tile is word (i & 1) * 16 + (j & 3) * 4 + (k' & 3) of
+// block ((i >> 1) * 4 + (j >> 2)) * kRotKB + (k' >> 2), so its bank is the triple
+// of digits (i & 1, j & 3, k' & 3).  The 4 x 4 x 4 stencil of any particle holds
+// every triple exactly twice (rows i and i + 2).  Lane l, which deposits a
+// particle of its own, therefore visits its 64 cells in an order of its own: at
+// step (ta, tb, tk) it adds the two cells whose digits are its lane's digits
+// plus (ta, tb, tk) (mod 2, 4, 4).  The 32 lanes of a warp have distinct digits,
+// so every one of the 64 atomics takes one shared-memory wavefront whatever the
+// particles' positions; only the weights and the address parts of each axis
+// have to be rotated, once per particle.  Random banks instead measured 2.6
+// cycles per atomic against 1.0.
+// k' = k + a shift of 0..3 chosen per row so that blocks of 4 k' are 16-byte
+// aligned in the grid, whose rows are Ng_pad floats apart: the write-out
+// then stores float4s.  A row's shift depends only on the tile and the row's
+// j parity (Ng even) and keeps the digits of a step distinct.
+// Cells outside the tile: along i two blocks on either side of the sums take
+// them and along k one more block (of both sides), none of which is read; along
+// j they get weight 0 and the block 0 cell of their digit.  A dense tile paints
+// 16 rows at a time into 64-bit sums of the same layout.
+// Bound by instruction issue (67 % of the slots at Ng = 512) and the barriers
+// between a tile's phases; 54 instructions per particle for both grids against
+// 94 of the staged deposit, 10 of them per-tile work.  Both grids of 1e8
+// uniform particles at Ng = 1024: 6.67 ms against 10.67; of the clustered 1e7 at
+// Ng = 512 with ten wedges, the whole call 3.31 ms against 3.73.
+constexpr int kRotKB = 10;                             // k' blocks of a row: 9 of the tile, 1 outside
+constexpr int kRotJB = kRotKB * 128;                   // bytes of one j block
+constexpr int kRotIB = 4 * kRotJB;                     // bytes of one i block (2 rows)
+constexpr int kRotJunk = 2;                            // i blocks below and above the tile
+constexpr size_t kRotAccBytes = (size_t)(16 + 2 * kRotJunk) * kRotIB;
+constexpr size_t kRotSmem = kRotAccBytes + 2 * kBlkN * sizeof(uint32_t);
+static_assert(16 / 2 * kRotIB * 2 <= (int)kRotAccBytes, "64-bit sums of 16 rows");
+static_assert(2 * (kRotSmem + 1280 + 1024) <= 228 * 1024, "two CTAs per SM");
+
+// first stencil cell (relative to the tile origin t0) and PCS weights (times
+// 6 s) along one axis of a record, in the grid shifted by delta (units of 2^-fb
+// cells).  A tile's particles have their first cell at -4 .. te (the base cell
+// of one grid lies up to one cell beyond the reach of the other's stencil); in
+// tiles at the box edge (fold) periodic images are folded there.
+__device__ __forceinline__ void record_axis(uint32_t rw, int delta, int fb, float inv, int Ng, int t0, bool fold,
+                                            float s, int &l, float w[4]) {
+    const uint32_t one = 1u << fb;
+    const int t = (int)(rw & (one - 1)) + delta;  // cell_g without its wrap
+    pcs_weights((float)((uint32_t)t & (one - 1)) * inv, w, s);
+    l = (int)(rw >> fb) + (t >> fb) - 1 - t0;
+    if (fold) {
+        l += l < -4 ? Ng : 0;
+        l -= l >= Ng - 4 ? Ng : 0;
+    }
+}
+
+// w[t] <- w[(t + r) & 3]
+__device__ __forceinline__ void rotate4(float w[4], int r) {
+    const bool r1 = r & 1, r2 = r & 2;
+    const float a = r1 ? w[1] : w[0], b = r1 ? w[2] : w[1], c = r1 ? w[3] : w[2], d = r1 ? w[0] : w[3];
+    w[0] = r2 ? c : a;
+    w[1] = r2 ? d : b;
+    w[2] = r2 ? a : c;
+    w[3] = r2 ? b : d;
+}
+
+// add the bits of v at byte address a + OFF of shared memory
+template <int OFF>
+__device__ __forceinline__ void red_shared(uint32_t a, float v) {
+    asm volatile("red.shared.add.u32 [%0+%2], %1;" ::"r"(a), "r"(__float_as_uint(v)), "n"(OFF) : "memory");
+}
+
+// (x, y) * (m, m), one packed instruction
+__device__ __forceinline__ void mul2(float x, float y, float m, float &px, float &py) {
+    asm("{\n .reg .b64 a, b, c;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %4};\n mul.rn.f32x2 c, a, b;\n mov.b64 {%0, %1}, c;\n}"
+        : "=f"(px), "=f"(py)
+        : "f"(x), "f"(y), "f"(m));
+}
+
+// what a CTA keeps for the tile it paints
+struct RotTile {
+    int t0[3], te[3];
+    int sh0, sh1;  // k shifts of the rows of even and odd local j
+    bool fold;     // the tile touches the box edge
+};
+
+// a lane's digits at steps 0 and 1 along j (in bytes: 16 each) and along k (4
+// each, in the rows of its own j parity); steps 2 and 3 are these with bit 1
+// flipped, and so are the rows of the other parity where the shifts differ
+struct RotLane {
+    int j0, j1, k0, k1, kflip;
+};
+
+// Deposit of one particle by its lane.  The products of the weights
+// are formed as denormal floats: w_ij is scaled by 2^-64 and w_k by 2^(s - 85), so
+// the FP32 multiplication itself rounds w_ij w_k 2^s to the nearest integer (its
+// bit pattern, below 2^24) and no conversion is left.
+__device__ __forceinline__ void rot_deposit(uint32_t acc, const uint4 &rec, int Ng, int fb, const RotTile &rt,
+                                            const RotLane &rl, const int delta[3], float inv, float s6k, int lane) {
+    const int lk = lane & 3, lb = (lane >> 2) & 3, la = lane >> 4;
+    constexpr float s6i = (1.f / 6.f) * 5.421010862427522e-20f;  // 2^-64 / 6
+    int li, lj, l0;
+    float wi[4], wj[4], wk[4];
+    record_axis(rec.x, delta[0], fb, inv, Ng, rt.t0[0], rt.fold, s6i, li, wi);
+    record_axis(rec.y, delta[1], fb, inv, Ng, rt.t0[1], rt.fold, 1.f / 6.f, lj, wj);
+    record_axis(rec.z, delta[2], fb, inv, Ng, rt.t0[2], rt.fold, s6k, l0, wk);
+    // the sums' i and k blocks cover first cells -4 .. te
+    if ((unsigned)(li + 4) > (unsigned)(rt.te[0] + 4) || (unsigned)(l0 + 4) > (unsigned)(rt.te[2] + 4)) return;
+    // i: rows of parity la, then 1 - la, each with the row 2 above it
+    const int ra = (la - li) & 1;
+    const int i0 = li + ra, i1 = li + 1 - ra;
+    const uint32_t ad_i0 = acc + (uint32_t)((i0 >> 1) * kRotIB + la * 64);
+    const uint32_t ad_i1 = acc + (uint32_t)((i1 >> 1) * kRotIB + (1 - la) * 64);
+    const float x00 = ra ? wi[1] : wi[0], x01 = ra ? wi[3] : wi[2];
+    const float x10 = ra ? wi[0] : wi[1], x11 = ra ? wi[2] : wi[3];
+    // j: the cells of digit D lie in block lj >> 2 if D >= lj & 3, else in the next
+    int ad_j[4];
+    {
+        const int f = (lj & 3) * 16, b0 = lj >> 2;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) wj[u] = (unsigned)(lj + u) < 16u ? wj[u] : 0.f;
+        rotate4(wj, (lb - lj) & 3);
+        const int base0 = (unsigned)b0 < 4u ? b0 * kRotJB : 0, base1 = (unsigned)(b0 + 1) < 4u ? (b0 + 1) * kRotJB : 0;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            const int D = ((t & 1) ? rl.j1 : rl.j0) ^ (t & 2 ? 32 : 0);
+            ad_j[t] = (D < f ? base1 : base0) + D;
+        }
+    }
+    // k: rows of the lane's own j parity (tb even) are shifted by shA, the others by shB
+    int ad_kA[4], ad_kB[4];
+    {
+        rotate4(wk, (lk - l0 - rt.sh0) & 3);
+        const int kA = l0 + ((lb & 1) ? rt.sh1 : rt.sh0), kB = l0 + ((lb & 1) ? rt.sh0 : rt.sh1);
+        const int fA = (kA & 3) * 4, fB = (kB & 3) * 4;
+        const int a1 = (kA >> 2) * 128 + 128, b1 = (kB >> 2) * 128 + 128;
+        const int a0 = kA < 0 ? 9 * 128 : a1 - 128, b0 = kB < 0 ? 9 * 128 : b1 - 128;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            const int DA = ((t & 1) ? rl.k1 : rl.k0) ^ (t & 2 ? 8 : 0), DB = DA ^ rl.kflip;
+            ad_kA[t] = (DA < fA ? a1 : a0) + DA;
+            ad_kB[t] = (DB < fB ? b1 : b0) + DB;
+        }
+    }
+#pragma unroll
+    for (int ta = 0; ta < 2; ++ta) {
+#pragma unroll
+        for (int tb = 0; tb < 4; ++tb) {
+            const uint32_t row = (ta ? ad_i1 : ad_i0) + (uint32_t)ad_j[tb];
+            float w0, w1;
+            mul2(ta ? x10 : x00, ta ? x11 : x01, wj[tb], w0, w1);
+#pragma unroll
+            for (int tk = 0; tk < 4; ++tk) {
+                const uint32_t a = row + (uint32_t)((tb & 1) ? ad_kB[tk] : ad_kA[tk]);
+                float p0, p1;
+                mul2(w0, w1, wk[tk], p0, p1);
+                red_shared<0>(a, p0);
+                red_shared<kRotIB>(a, p1);
+            }
+        }
+    }
+}
+
+// the same into the 64-bit sums of rows [h, h + rows) of a dense tile
+__device__ __forceinline__ void rot_deposit_wide(unsigned long long *acc, const uint4 &rec, int Ng, int fb,
+                                                 const RotTile &rt, int h, int rows, const int delta[3], float inv,
+                                                 float kscale) {
+    int l[3];
+    float w[3][4];
+    record_axis(rec.x, delta[0], fb, inv, Ng, rt.t0[0], true, 1.f / 6.f, l[0], w[0]);
+    record_axis(rec.y, delta[1], fb, inv, Ng, rt.t0[1], true, 1.f / 6.f, l[1], w[1]);
+    record_axis(rec.z, delta[2], fb, inv, Ng, rt.t0[2], true, 1.f / 6.f, l[2], w[2]);
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        const int i = l[0] + a - h;
+        if ((unsigned)i >= (unsigned)rows) continue;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const int j = l[1] + b;
+            if ((unsigned)j >= (unsigned)rt.te[1]) continue;
+            const float wij = (w[0][a] * 5.421010862427522e-20f) * w[1][b];
+            const int sh = (j & 1) ? rt.sh1 : rt.sh0;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int k = l[2] + c;
+                if ((unsigned)k >= (unsigned)rt.te[2]) continue;
+                const int kp = k + sh;
+                atomicAdd(acc + (((i >> 1) * 4 + (j >> 2)) * kRotKB + (kp >> 2)) * 32 + (i & 1) * 16 + (j & 3) * 4 +
+                              (kp & 3),
+                          (unsigned long long)__float_as_uint(wij * (w[2][c] * kscale)));
+            }
+        }
+    }
+}
+
+// Persistent like paint_coop_kernel.  split: even CTAs paint grid 0 and odd
+// CTAs grid 1 of the same tiles, from one sort keyed for both grids.  The
+// offsets of the next tile's segments are loaded before the deposits and its
+// first records before the write-out, so their latencies hide behind them.
+__global__ void __launch_bounds__(kPaintThreads, 2)
+paint_rot_kernel(PaintParams pp, const uint32_t *__restrict__ off, const uint4 *__restrict__ sorted, PaintOut po,
+                 unsigned ntiles, int split) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    unsigned char *accb = smem_raw + kRotJunk * kRotIB;  // the tile's block 0
+    uint32_t *blk = reinterpret_cast<uint32_t *>(smem_raw + kRotAccBytes);
+    __shared__ uint32_t seg_begin[128];
+    __shared__ uint32_t seg_pref[128 + 1];
+    __shared__ uint32_t scan_ws[33];
+    __shared__ int fixbits_s;
+    __shared__ int geo[6];         // t0, te of the tile
+    __shared__ uint32_t first[2];  // the next tile's own particles: first record, count
+    const int Ng = pp.Ng, fb = pp.fb, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int nwarp = kPaintThreads / 32;
+    const int g = split ? (int)(blockIdx.x & 1) : 0;
+    const int delta[3] = {g ? pp.ax[0].dq[1] : pp.ax[0].dq[0], g ? pp.ax[1].dq[1] : pp.ax[1].dq[0],
+                          g ? pp.ax[2].dq[1] : pp.ax[2].dq[0]};
+    float *const out = reinterpret_cast<float *>(g ? po.out[1] : po.out[0]);
+    const double scd = po.ds ? po.ds->scale[g] : (g ? po.scale[1] : po.scale[0]);
+    const float scf = (float)scd;
+    const int accu = g ? po.accumulate[1] : po.accumulate[0];
+    const unsigned cta = split ? blockIdx.x >> 1 : blockIdx.x;
+    const unsigned ncta = split ? gridDim.x >> 1 : gridDim.x;
+    unsigned tile = cta;
+    if (tile >= ntiles) return;
+    for (int e = tid; e < (int)(kRotAccBytes / 16); e += kPaintThreads)
+        reinterpret_cast<uint4 *>(smem_raw)[e] = make_uint4(0, 0, 0, 0);
+    // the segments of a tile, one per thread of the first four warps, and its
+    // geometry, loaded into registers that nothing reads until publish() ...
+    uint32_t nb_begin = 0, nb_end = 0;
+    int nb_t0 = 0, nb_t1 = 0;
+    const int nt0 = pp.nt[0], nt1 = pp.nt[1], nt2 = pp.nt[2];
+    // thread q's segment as an offset from the tile and a class, the options
+    // per axis as in tile_segment (two tiles or more along every axis)
+    int sd[3] = {0, 0, 0}, scls = 0, scnt = tid == 0 ? 27 : (tid < kMaxSeg ? 1 : 0);
+    if (tid > 0 && tid < kMaxSeg) {
+        const int idx[3] = {tid / 25, (tid / 5) % 5, tid % 5};
+        bool own = true;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const int x = idx[a], nt = pp.nt[a];
+            int c = x;
+            if (x >= 3) {
+                own = false;
+                sd[a] = nt > 2 && x == 3 ? -1 : 1;
+                c = (x == 3) == (nt > 2) ? 2 : 1;
+            }
+            scls = 3 * scls + c;
+        }
+        if (own) scnt = 0;  // part of segment 0
+    }
+    auto fetch = [&](unsigned t) {
+        if (warp >= 4) return;
+        const unsigned ti = t / (unsigned)nt2, tk = t - ti * nt2, t0i = ti / (unsigned)nt1, tj = ti - t0i * nt1;
+        int o0 = (int)t0i + sd[0], o1 = (int)tj + sd[1], o2 = (int)tk + sd[2];
+        o0 = o0 < 0 ? o0 + nt0 : (o0 >= nt0 ? o0 - nt0 : o0);
+        o1 = o1 < 0 ? o1 + nt1 : (o1 >= nt1 ? o1 - nt1 : o1);
+        o2 = o2 < 0 ? o2 + nt2 : (o2 >= nt2 ? o2 - nt2 : o2);
+        const uint32_t key = (uint32_t)((o0 * nt1 + o1) * nt2 + o2) * 27u + (uint32_t)scls;
+        nb_begin = off[key];
+        nb_end = off[key + (uint32_t)scnt];
+        if (tid < 3) {
+            const int *st = pp.start[tid];
+            const unsigned q = tid == 0 ? t0i : tid == 1 ? tj : tk;
+            nb_t0 = st[q];
+            nb_t1 = st[q + 1];
+        }
+    };
+    // ... and published in shared memory with the counts' prefix sums
+    auto publish = [&]() {
+        const uint32_t nb_cnt = nb_end - nb_begin;
+        uint32_t inc = nb_cnt;
+        if (warp < 4) {
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += u;
+            }
+            if (lane == 31) scan_ws[warp] = inc;
+            if (tid < 3) {
+                geo[tid] = nb_t0;
+                geo[3 + tid] = nb_t1 - nb_t0;
+            }
+        }
+        __syncthreads();
+        if (warp < 4) {
+            uint32_t add = 0;
+            for (int w = 0; w < warp; ++w) add += scan_ws[w];
+            seg_begin[tid] = nb_begin;
+            seg_pref[tid] = add + inc - nb_cnt;
+            if (tid == 127) seg_pref[128] = add + inc;
+        }
+        __syncthreads();
+    };
+    fetch(tile);
+    publish();  // also orders the clearing above
+    constexpr int nseg = 128;  // segments 125 .. 127 are empty
+    uint4 rec = make_uint4(0, 0, 0, 0);
+    if ((uint32_t)tid < seg_pref[1]) rec = sorted[seg_begin[0] + tid];
+    const float inv = __int_as_float((127 - fb) << 23);  // 2^-fb (fb <= 24)
+    const uint32_t acc = (uint32_t)__cvta_generic_to_shared(accb);
+    const bool flip = (pp.Ng_pad & 3) != 0;        // rows alternate between 16-byte alignment and 8 off it
+    const bool vec = !flip || (Ng & 1) == 0;       // the shift depends on j alone
+    const long rstride = (long)pp.Ng_pad, istride = rstride * Ng;
+    RotLane rl;
+    {
+        const int lk = lane & 3, lb = (lane >> 2) & 3;
+        rl.kflip = vec && flip ? 8 : 0;
+        rl.j0 = lb * 16;
+        rl.j1 = ((lb + 1) & 3) * 16;
+        rl.k0 = (lk * 4) ^ ((lb & 1) ? rl.kflip : 0);
+        rl.k1 = (((lk + 1) & 3) * 4) ^ ((lb & 1) ? rl.kflip : 0);
+    }
+    for (;;) {
+        const uint32_t total = seg_pref[128];
+        RotTile rt;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            rt.t0[a] = geo[a];
+            rt.te[a] = geo[3 + a];
+        }
+        rt.fold = rt.t0[0] == 0 || rt.t0[1] == 0 || rt.t0[2] == 0 || rt.t0[0] + rt.te[0] == Ng ||
+                  rt.t0[1] + rt.te[1] == Ng || rt.t0[2] + rt.te[2] == Ng;
+        rt.sh0 = rt.sh1 = 0;
+        if (vec) {
+            rt.sh0 = (rt.t0[2] + (flip ? 2 * rt.t0[1] : 0)) & 3;
+            rt.sh1 = (rt.t0[2] + (flip ? 2 * (rt.t0[1] + 1) : 0)) & 3;
+        }
+        const unsigned next = tile + ncta;
+        if (next < ntiles) fetch(next);
+        const uint32_t own = seg_pref[1];  // segment 0: the tile's own particles
+        auto index = [&](uint32_t q) -> uint32_t {
+            return q < own ? seg_begin[0] + q : seg_index(q, seg_begin, seg_pref, nseg);
+        };
+        int fixbits = fix_bits_for(total);
+        if (fixbits < kBlockCountBelow) {
+            const bool cyc[3] = {false, false, false};  // Ng >= 64: two tiles or more along every axis
+            TileSegs ts;
+            for (int a = 0; a < 3; ++a) ts.t0[a] = rt.t0[a];
+            fixbits = tile_fixbits(total, sorted, index, pp, ts, cyc, blk, blk + kBlkN, scan_ws, &fixbits_s);
+        }
+        const bool wide = fixbits < kWideBelow;
+        const int te0 = rt.te[0], te1 = rt.te[1], te2 = rt.te[2];
+        const int rowlen = te2 + (rt.t0[2] + te2 == Ng ? pp.Ng_pad - Ng : 0);  // with the padding of the last k tile
+        float *obase = out + ((long)rt.t0[0] * Ng + rt.t0[1]) * rstride + rt.t0[2];
+        if (!wide) {
+            const float s6k = (1.f / 6.f) * __int_as_float((127 + fixbits - 85) << 23);  // 2^(s - 85) / 6
+            if ((uint32_t)tid >= own && (uint32_t)tid < total) rec = sorted[index((uint32_t)tid)];
+            for (uint32_t q = tid; q < total; q += kPaintThreads) {
+                const uint4 r = rec;
+                if (q + kPaintThreads < total) rec = sorted[index(q + kPaintThreads)];  // in flight during the deposit
+                rot_deposit(acc, r, Ng, fb, rt, rl, delta, inv, s6k, lane);
+            }
+            if (tid == 0) {
+                first[0] = nb_begin;
+                first[1] = next < ntiles ? nb_end - nb_begin : 0u;
+            }
+            __syncthreads();
+            if ((uint32_t)tid < first[1]) rec = sorted[first[0] + tid];
+            // write the owned cells and clear the sums.  A warp takes a block row (2 x 4
+            // rows): 8 lanes read the 8 rows of one block (one wavefront), the four
+            // groups of 8 lanes blocks kq and kq + 4 along k; then lanes l and l ^ 4
+            // exchange so that a store covers 4 whole rows of the tile.  (64-byte
+            // pieces of 8 rows took 18 store wavefronts per instruction, and the
+            // whole paint 7.36 ms.)
+            const float sc = scf * __int_as_float((127 - fixbits) << 23);  // scale 2^-s
+            const float padv = 0.f * sc;  // padding cells take 0 x scale, as the reference
+                                          // scales the whole padded grid (src/fft.c:127-129)
+            // shift, extent and padding are even and the rows 16-byte aligned up to their shift
+            const bool pairs = vec && !accu && ((rt.sh0 | te2 | rowlen) & 1) == 0;
+            static_assert(nwarp == 16, "a warp's block rows are 8 rows apart, with one j");
+            const int r = lane & 7, kq = lane >> 3, hi = r >> 2;
+            const int j = 4 * (warp & 3) + (r & 3), sh = (r & 1) ? rt.sh1 : rt.sh0;
+            const int k = 4 * (kq + 4 * hi) - sh;  // after the exchange
+            const bool full = pairs && te0 == 32 && te1 == 16 && rowlen == 32;  // no checks but the ends of shifted rows
+            int i = 2 * (warp >> 2);
+            uint4 *src = reinterpret_cast<uint4 *>(accb) + (warp * kRotKB + kq) * 8 + r;
+            float *o = obase + i * istride + j * rstride + k;
+            const long tail_off = (hi ? istride - 16 : 0) + 32;  // o is at block 4 hi of row i
+            auto take = [&](uint4 *sp) {
+                const uint4 c = *sp;
+                *sp = make_uint4(0, 0, 0, 0);
+                return make_float4(__uint2float_rn(c.x) * sc, __uint2float_rn(c.y) * sc, __uint2float_rn(c.z) * sc,
+                                   __uint2float_rn(c.w) * sc);
+            };
+            // cells kk .. kk + 3 of a row of the tile
+            auto put = [&](float *op, const float4 &u, int kk) {
+                if (pairs && kk >= 0 && kk + 4 <= te2) {
+                    *reinterpret_cast<float4 *>(op) = u;
+                } else if (pairs) {
+                    // the ends of a row: kk, te2 and rowlen are even
+                    if ((unsigned)kk < (unsigned)rowlen)
+                        *reinterpret_cast<float2 *>(op) = kk < te2 ? make_float2(u.x, u.y) : make_float2(padv, padv);
+                    if ((unsigned)(kk + 2) < (unsigned)rowlen)
+                        *reinterpret_cast<float2 *>(op + 2) =
+                            kk + 2 < te2 ? make_float2(u.z, u.w) : make_float2(padv, padv);
+                } else {
+                    const float v[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        if ((unsigned)(kk + q) >= (unsigned)rowlen) continue;
+                        if (!accu) op[q] = kk + q < te2 ? v[q] : padv;
+                        else if (kk + q < te2) op[q] += v[q];
+                    }
+                }
+            };
+            for (int m = 0; m < 4; ++m, i += 8, src += nwarp * kRotKB * 8, o += 8 * istride) {
+                float4 u = take(src), v = take(src + 4 * 8);
+                const float4 snd = hi ? u : v;
+                float4 rcv;
+                rcv.x = __shfl_xor_sync(0xffffffffu, snd.x, 4);
+                rcv.y = __shfl_xor_sync(0xffffffffu, snd.y, 4);
+                rcv.z = __shfl_xor_sync(0xffffffffu, snd.z, 4);
+                rcv.w = __shfl_xor_sync(0xffffffffu, snd.w, 4);
+                if (hi) u = rcv;  // row i, blocks kq + 4 hi
+                else v = rcv;     // row i + 1
+                if (full) {
+                    if (k >= 0) {
+                        *reinterpret_cast<float4 *>(o) = u;
+                        *reinterpret_cast<float4 *>(o + istride) = v;
+                    } else {
+                        *reinterpret_cast<float2 *>(o + 2) = make_float2(u.z, u.w);
+                        *reinterpret_cast<float2 *>(o + istride + 2) = make_float2(v.z, v.w);
+                    }
+                } else if (j < te1) {
+                    if (i < te0) put(o, u, k);
+                    if (i + 1 < te0) put(o + istride, v, k);
+                }
+                if (kq == 0) {  // block 8 of row i + hi: the last cells of the shifted rows, and the padding
+                    float *ot = o + tail_off;
+                    const float4 w = take(src + 8 * 8);
+                    if (full) {
+                        if (sh) *reinterpret_cast<float2 *>(ot) = make_float2(w.x, w.y);
+                    } else if (j < te1 && i + hi < te0) {
+                        put(ot, w, 32 - sh);
+                    }
+                }
+            }
+        } else {
+            // 16 rows at a time in 64-bit sums
+            const float kscale = __int_as_float((127 + kWideBits - 85) << 23);
+            const double sc = ldexp(scd, -kWideBits);
+            unsigned long long *acc64 = reinterpret_cast<unsigned long long *>(smem_raw);
+            for (int h = 0; h < te0; h += 16) {
+                const int rows = min(16, te0 - h);
+                __syncthreads();
+                for (int e = tid; e < (int)(kRotAccBytes / 16); e += kPaintThreads)
+                    reinterpret_cast<uint4 *>(smem_raw)[e] = make_uint4(0, 0, 0, 0);
+                __syncthreads();
+                for (uint32_t q = tid; q < total; q += kPaintThreads)
+                    rot_deposit_wide(acc64, sorted[index(q)], Ng, fb, rt, h, rows, delta, inv, kscale);
+                __syncthreads();
+                for (int b = warp; b < 8 * 4 * kRotKB; b += nwarp) {
+                    const int kb = b % kRotKB, rowb = b / kRotKB;
+                    const int i = 2 * (rowb >> 2) + (lane >> 4), j = 4 * (rowb & 3) + ((lane >> 2) & 3);
+                    const int k = 4 * kb + (lane & 3) - ((j & 1) ? rt.sh1 : rt.sh0);
+                    if (i >= rows || j >= te1 || (unsigned)k >= (unsigned)rowlen) continue;
+                    float *o = obase + (h + i) * istride + j * rstride + k;
+                    const float v = (float)((double)acc64[b * 32 + lane] * sc);
+                    if (!accu) *o = v;
+                    else if (k < te2) *o += v;
+                }
+            }
+            if (tid == 0) {
+                first[0] = nb_begin;
+                first[1] = next < ntiles ? nb_end - nb_begin : 0u;
+            }
+            __syncthreads();
+            if ((uint32_t)tid < first[1]) rec = sorted[first[0] + tid];
+            for (int e = tid; e < (int)(kRotAccBytes / 16); e += kPaintThreads)
+                reinterpret_cast<uint4 *>(smem_raw)[e] = make_uint4(0, 0, 0, 0);
+        }
+        if (next >= ntiles) break;
+        publish();  // the clearing above completes before the next deposit
         tile = next;
     }
 }
@@ -1269,25 +1733,27 @@ int paint(const PaintTiling *t, PaintScratch *s, int grid_prec, const void *x, c
     if (ev) FG_CUDA(cudaEventRecord(ev[2], st));
     const unsigned ntiles = (unsigned)((long)t->nt[0] * t->nt[1] * t->nt[2]);
     if (grid_prec == 4) {
-        // one grid per CTA where the tiles are 32 x 16 x 32: with two grids,
-        // even CTAs paint grid 0 and odd CTAs grid 1 (the sort's keys cover
-        // both grids' stencils); else both grids of 16-row tiles per CTA
-        constexpr int T = kPaintThreads;
-        const size_t smem = kAccBytes + sizeof(StageBuf) * (T / 32);
-        FG_CUDA(cudaFuncSetAttribute(paint_coop_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        FG_CUDA(cudaFuncSetAttribute(paint_coop_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        const int split = big && ngrids == 2;
-        unsigned nb = (unsigned)((cta_per_sm == 1 ? 1 : 2) * num_sms());
-        if (split) {
-            nb = nb < 2 * ntiles ? nb : 2 * ntiles;
-            nb &= ~1u;
+        const unsigned slots = (unsigned)((cta_per_sm == 1 ? 1 : 2) * num_sms());
+        if (big) {
+            // one grid per CTA: with two grids, even CTAs paint grid 0 and odd
+            // CTAs grid 1 (the sort's keys cover both grids' stencils)
+            const int split = ngrids == 2;
+            unsigned nb = slots < ntiles * ngrids ? slots : ntiles * ngrids;
+            if (split) nb &= ~1u;
+            FG_CUDA(cudaFuncSetAttribute(paint_rot_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRotSmem));
+            paint_rot_kernel<<<nb, kPaintThreads, kRotSmem, st>>>(pp, s->hist, (const uint4 *)s->sorted, po, ntiles,
+                                                                  split);
         } else {
-            nb = nb < ntiles ? nb : ntiles;
+            constexpr int T = kPaintThreads;
+            const size_t smem = kAccBytes + sizeof(StageBuf) * (T / 32);
+            const unsigned nb = slots < ntiles ? slots : ntiles;
+            FG_CUDA(cudaFuncSetAttribute(paint_coop_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            FG_CUDA(cudaFuncSetAttribute(paint_coop_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            if (ngrids == 1)
+                paint_coop_kernel<1><<<nb, T, smem, st>>>(pp, s->hist, (const uint4 *)s->sorted, po, ntiles);
+            else
+                paint_coop_kernel<2><<<nb, T, smem, st>>>(pp, s->hist, (const uint4 *)s->sorted, po, ntiles);
         }
-        if (ngrids == 1 || split)
-            paint_coop_kernel<1><<<nb, T, smem, st>>>(pp, s->hist, (const uint4 *)s->sorted, po, ntiles, split);
-        else
-            paint_coop_kernel<2><<<nb, T, smem, st>>>(pp, s->hist, (const uint4 *)s->sorted, po, ntiles, 0);
     } else {
         const size_t smem = (size_t)ngrids * kT3 * sizeof(double);
         FG_CUDA(cudaFuncSetAttribute(paint_tile_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
