@@ -694,8 +694,7 @@ extern "C" void fft_x2k(fft_t *self, int offset_phase_on) {
     Grid *g = G(self);
     FG_API(enter(self, true), "fft_x2k()");
     void *grids[1] = {g->d_f};
-    FG_API(fft_r2c(&g->fft, grids, 1, g->stream), "fft_x2k()");
-    FG_API(scale_grid(g->d_f, self->Ng3_pad, g->prec, H3_of(g), g->stream), "fft_x2k()");
+    FG_API(fft_r2c(&g->fft, grids, 1, g->stream, H3_of(g)), "fft_x2k()");
     if (offset_phase_on) FG_API(phase(g, g->d_f, self->offset, 1), "fft_x2k()");
     FG_API(leave(self, true), "fft_x2k()");
     if (!g->quiet) fprintf(stderr, "fft_x2k() %.2fs\n", now_s() - t);
@@ -706,9 +705,8 @@ extern "C" void fft_k2x(fft_t *self, int offset_phase_off) {
     Grid *g = G(self);
     FG_API(enter(self, true), "fft_k2x()");
     void *grids[1] = {g->d_f};
-    FG_API(fft_c2r(&g->fft, grids, 1, g->stream), "fft_k2x()");
     const double L3 = self->L * self->L * self->L;
-    FG_API(scale_grid(g->d_f, self->Ng3_pad, g->prec, 1 / L3, g->stream), "fft_k2x()");
+    FG_API(fft_c2r(&g->fft, grids, 1, g->stream, 1 / L3), "fft_k2x()");
     if (offset_phase_off) FG_API(phase(g, g->d_f, self->offset, -1), "fft_k2x()");
     FG_API(leave(self, true), "fft_k2x()");
     if (!g->quiet) fprintf(stderr, "fft_k2x() %.2fs\n", now_s() - t);
@@ -1391,8 +1389,7 @@ extern "C" int fftgal_dl_sub(fft_t *grid, int sphere, int Nsub, int nlos, const 
         hat(lh);
         for (int iL = 0; iL < 3 && rc == OK; ++iL) {
             rc = dl_filter(g->d_f, g->d_aux, Ng, g->prec, sphere, d_tab, lh, iL, st);
-            if (rc == OK) rc = fft_c2r(&g->fft, grids, 1, st);
-            if (rc == OK) rc = scale_grid(g->d_f, grid->Ng3_pad, g->prec, 1 / L3, st);
+            if (rc == OK) rc = fft_c2r(&g->fft, grids, 1, st, 1 / L3);
             if (rc == OK) rc = dl_sample(g->d_f, Ng, g->prec, Nsub, bias, d_out + (size_t)(3 * l + iL) * nsub3, st);
         }
     }

@@ -509,10 +509,25 @@ static void launch_k(bool forward, dim3 grid, const FftPlan *p, void *g0, void *
                                                                          p->rows, d, (const T2 *)p->rtw);
 }
 
-static int k_pass(const FftPlan *p, void *const *grids, int ngrids, bool forward, cudaStream_t s) {
+// the general kernels leave the normalisation to a pass of its own (FP64 grids
+// keep the reference's order of operations)
+static int scale_grids(const FftPlan *p, void *const *grids, int ngrids, double scale, cudaStream_t s) {
+    if (scale == 1) return OK;
+    for (int q = 0; q < ngrids; ++q)
+        FG_TRY(scale_grid(grids[q], 2L * p->Ng * p->Ng * p->nh, p->prec, scale, s));
+    return OK;
+}
+
+// The k pass: forward, powers of two take fft2.cu's packed rows (half-length
+// transforms); everything else, and every backward pass, the row pairs of
+// fft3.cu where the length splits; the general kernels below otherwise (c2r
+// at Ng = 512: 733 us there, at Ng = 384 both grids forward 1402 us).
+static int k_pass(const FftPlan *p, void *const *grids, int ngrids, bool forward, cudaStream_t s, double scale = 1) {
     if (forward && fft2_supported(p->Ng, p->prec))
         return fft2_k_r2c(p->Ng, p->half.tw, p->rtw, grids[0], ngrids > 1 ? grids[1] : grids[0], ngrids, s,
                           p->tune[0]);
+    if (fft3_supported(p->Ng, p->prec))
+        return fft3_k(p->Ng, p->axis.tw, grids[0], ngrids > 1 ? grids[1] : grids[0], ngrids, forward, scale, s);
     const long nrows = (long)p->Ng * p->Ng;
     const Fft1dPlan &kp = p->even ? p->half : p->axis;
     const Fft1dDev d = to_dev(kp);
@@ -527,7 +542,7 @@ static int k_pass(const FftPlan *p, void *const *grids, int ngrids, bool forward
         else launch_k<double, false>(forward, grid, p, grids[0], g1, nrows, d, s);
     }
     FG_LAUNCHED(1);
-    return OK;
+    return scale_grids(p, grids, ngrids, scale, s);
 }
 
 int fft_pass_k_r2c(const FftPlan *p, void *const *grids, int ngrids, cudaStream_t s) {
@@ -543,10 +558,13 @@ static void launch_cols(dim3 grid, const FftPlan *p, void *g0, void *g1, long el
 }
 
 static int cols_pass(const FftPlan *p, void *const *grids, int ngrids, int sign,
-                     long elem_stride, long batch_stride, cudaStream_t s, int logC) {
+                     long elem_stride, long batch_stride, cudaStream_t s, int logC, double scale = 1) {
     if (fft2_supported(p->Ng, p->prec))
         return fft2_cols(p->Ng, p->axis.tw, grids[0], ngrids > 1 ? grids[1] : grids[0], ngrids, p->nh,
-                         elem_stride, batch_stride, p->Ng, sign, s, logC);
+                         elem_stride, batch_stride, p->Ng, sign, s, logC, scale);
+    if (fft3_supported(p->Ng, p->prec))
+        return fft3_cols(p->Ng, p->axis.tw, grids[0], ngrids > 1 ? grids[1] : grids[0], ngrids, p->nh, elem_stride,
+                         batch_stride, p->Ng, sign, scale, s);
     const Fft1dDev d = to_dev(p->axis);
     const long ncb = ceil_div(p->nh, p->cols);
     dim3 grid((unsigned)(ncb * p->Ng), ngrids);
@@ -560,30 +578,31 @@ static int cols_pass(const FftPlan *p, void *const *grids, int ngrids, int sign,
         else launch_cols<double, false>(grid, p, grids[0], g1, elem_stride, batch_stride, d, sign, s);
     }
     FG_LAUNCHED(1);
-    return OK;
+    return scale_grids(p, grids, ngrids, scale, s);
 }
 
 int fft_pass_j(const FftPlan *p, void *const *grids, int ngrids, int sign, cudaStream_t s) {
     return cols_pass(p, grids, ngrids, sign, p->nh, (long)p->Ng * p->nh, s, p->tune[1]);
 }
 
-int fft_pass_i(const FftPlan *p, void *const *grids, int ngrids, int sign, cudaStream_t s) {
-    if (fft2_tma_supported(p->Ng, p->prec))
-        return fft2_cols_tma(p->Ng, p->axis.tw, grids[0], ngrids > 1 ? grids[1] : grids[0], ngrids, sign, s);
-    return cols_pass(p, grids, ngrids, sign, (long)p->Ng * p->nh, p->nh, s, p->tune[2]);
+int fft_pass_i(const FftPlan *p, void *const *grids, int ngrids, int sign, cudaStream_t s, double scale) {
+    if (fft2_tma_supported(p->Ng, p->prec)) {
+        FG_TRY(fft2_cols_tma(p->Ng, p->axis.tw, grids[0], ngrids > 1 ? grids[1] : grids[0], ngrids, sign, s));
+        return scale_grids(p, grids, ngrids, scale, s);
+    }
+    return cols_pass(p, grids, ngrids, sign, (long)p->Ng * p->nh, p->nh, s, p->tune[2], scale);
 }
 
-int fft_r2c(const FftPlan *p, void *const *grids, int ngrids, cudaStream_t s) {
+int fft_r2c(const FftPlan *p, void *const *grids, int ngrids, cudaStream_t s, double scale) {
     FG_TRY(fft_pass_k_r2c(p, grids, ngrids, s));
     FG_TRY(fft_pass_j(p, grids, ngrids, -1, s));
-    FG_TRY(fft_pass_i(p, grids, ngrids, -1, s));
-    return OK;
+    return fft_pass_i(p, grids, ngrids, -1, s, scale);
 }
 
-int fft_c2r(const FftPlan *p, void *const *grids, int ngrids, cudaStream_t s) {
+int fft_c2r(const FftPlan *p, void *const *grids, int ngrids, cudaStream_t s, double scale) {
     FG_TRY(fft_pass_i(p, grids, ngrids, +1, s));
     FG_TRY(fft_pass_j(p, grids, ngrids, +1, s));
-    return k_pass(p, grids, ngrids, false, s);
+    return k_pass(p, grids, ngrids, false, s, scale);
 }
 
 }  // namespace fg

@@ -14,8 +14,8 @@
 // phases are free of bank conflicts.  Length 2048 on the strided axes is
 // 32 x 64 with the 64-point second step split over lane pairs
 // (fft2_cols2048_kernel).  Used for the forward r2c k pass and the strided
-// j/i passes of FP32 grids; other lengths and FP64 grids use the general
-// kernels of fft.cu.
+// j/i passes of FP32 grids; other lengths use fft3.cu's mixed-radix passes or,
+// where those do not apply (FP64 grids among them), the general kernels of fft.cu.
 #include "internal.h"
 #include "common.cuh"
 
@@ -76,13 +76,21 @@ __device__ __forceinline__ float2 twid(const float2 *__restrict__ W, int t, int 
     return w;
 }
 
+// the last pass of a transform applies its normalisation while storing
+template <int M>
+__device__ __forceinline__ void scale_all(float2 (&v)[M], float scale) {
+    if (scale == 1.f) return;
+#pragma unroll
+    for (int i = 0; i < M; ++i) v[i] = make_float2(v[i].x * scale, v[i].y * scale);
+}
+
 // ---- strided axis: C columns per CTA, threads = C * N2 ---------------------------
 // element n of column c of batch b: base + b*bs + n*es + c0 + c (complex units)
 // One tile: columns c0 .. c0 + C - 1 at `base` (= g + b*bs + c0), `left`
 // columns of them valid; threads t < nthr of the CTA (nthr >= C*N2).
 template <int N1, int N2>
 __device__ __forceinline__ void cols_tile(float2 *base, int left, long es, int logC, const float2 *__restrict__ W,
-                                          int sign, float2 *S, int t, int nthr) {
+                                          int sign, float scale, float2 *S, int t, int nthr) {
     const int C = 1 << logC;
     const int P = N1 * C + 8;  // shared pitch per n2
     if (t < C * N2) {
@@ -102,6 +110,7 @@ __device__ __forceinline__ void cols_tile(float2 *base, int left, long es, int l
 #pragma unroll
             for (int k1 = 0; k1 < N1; ++k1) S[n2 * P + k1 * C + c] = v[k1];
         } else {
+            scale_all<N1>(v, scale);
             if (ok)
 #pragma unroll
                 for (int k1 = 0; k1 < N1; ++k1) base[(long)k1 * es + c] = v[k1];
@@ -115,6 +124,7 @@ __device__ __forceinline__ void cols_tile(float2 *base, int left, long es, int l
 #pragma unroll
             for (int n2 = 0; n2 < N2; ++n2) u[n2] = S[n2 * P + k1 * C + c];
             reg_fft<N2>(u, sign);
+            scale_all<N2>(u, scale);
             if (c < left)
 #pragma unroll
                 for (int k2 = 0; k2 < N2; ++k2) base[(long)(k1 + N1 * k2) * es + c] = u[k2];
@@ -125,7 +135,7 @@ __device__ __forceinline__ void cols_tile(float2 *base, int left, long es, int l
 template <int N1, int N2>
 __global__ void __launch_bounds__(512)
 fft2_cols_kernel(float2 *g0, float2 *g1, int ncols, long es, long bs, int logC,
-                 const float2 *__restrict__ W, int sign) {
+                 const float2 *__restrict__ W, int sign, float scale) {
     extern __shared__ __align__(16) float2 S[];
     const int C = 1 << logC;
     const int ncb = (ncols + C - 1) >> logC;
@@ -133,7 +143,7 @@ fft2_cols_kernel(float2 *g0, float2 *g1, int ncols, long es, long bs, int logC,
     const long batch = blockIdx.x / ncb;
     float2 *g = blockIdx.y == 0 ? g0 : g1;
     const int c0 = cb << logC;
-    cols_tile<N1, N2>(g + batch * bs + c0, ncols - c0, es, logC, W, sign, S, threadIdx.x, blockDim.x);
+    cols_tile<N1, N2>(g + batch * bs + c0, ncols - c0, es, logC, W, sign, scale, S, threadIdx.x, blockDim.x);
 }
 
 // ---- strided axis of length 2048 = 32 x 64 ---------------------------------------------
@@ -147,7 +157,7 @@ fft2_cols_kernel(float2 *g0, float2 *g1, int ncols, long es, long bs, int logC,
 // 32 distinct banks; the step-1 stores then take two wavefronts.
 __global__ void __launch_bounds__(512)
 fft2_cols2048_kernel(float2 *g0, float2 *g1, int ncols, long es, long bs, int logC, const float2 *__restrict__ W,
-                     int sign) {
+                     int sign, float scale) {
     constexpr int N1 = 32, N2 = 64;
     extern __shared__ __align__(16) float2 S[];
     const int C = 1 << logC;
@@ -190,7 +200,8 @@ fft2_cols2048_kernel(float2 *g0, float2 *g1, int ncols, long es, long bs, int lo
         other.y = __shfl_xor_sync(0xffffffffu, u[k2].y, 16);
         const float2 E = h ? other : u[k2], O = h ? u[k2] : other;
         const float2 wo = cmul(O, twid(W, 32 * k2, sign));  // W_2048^(32 k2) = W_64^k2
-        const float2 x = h ? csub(E, wo) : cadd(E, wo);
+        float2 x = h ? csub(E, wo) : cadd(E, wo);
+        if (scale != 1.f) x = make_float2(x.x * scale, x.y * scale);
         if (ok) base[(long)(k1 + N1 * (k2 + 32 * h)) * es + c] = x;
     }
 }
@@ -630,7 +641,7 @@ bool fft2_supported(int Ng, int prec) {
         FG_CUDA(cudaFuncSetAttribute(fft2_cols_kernel<A, B>, cudaFuncAttributeMaxDynamicSharedMemorySize,   \
                                      (int)smem));                                                         \
         fft2_cols_kernel<A, B><<<grid, threads, smem, s>>>((float2 *)g0, (float2 *)g1, ncols, es, bs,      \
-                                                           logC, (const float2 *)W, sign);                 \
+                                                           logC, (const float2 *)W, sign, (float)scale);   \
         FG_LAUNCHED(1);                                                                                    \
         return OK;                                                                                         \
     }
@@ -804,7 +815,7 @@ int fft2_tma_check() {
 }
 
 int fft2_cols(int N, const void *W, void *g0, void *g1, int ngrids, int ncols, long es, long bs,
-              long nbatch, int sign, cudaStream_t s, int logC_req) {
+              long nbatch, int sign, cudaStream_t s, int logC_req, double scale) {
     FG_TRY(ensure_w32());
     int N1, N2;
     bool paired;
@@ -825,7 +836,7 @@ int fft2_cols(int N, const void *W, void *g0, void *g1, int ngrids, int ncols, l
     if (paired) {
         FG_CUDA(cudaFuncSetAttribute(fft2_cols2048_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         fft2_cols2048_kernel<<<grid, threads, smem, s>>>((float2 *)g0, (float2 *)g1, ncols, es, bs, logC,
-                                                         (const float2 *)W, sign);
+                                                         (const float2 *)W, sign, (float)scale);
         FG_LAUNCHED(1);
         return OK;
     }

@@ -77,19 +77,19 @@ struct FftPlan {
 
 int fft_plan_create(FftPlan *p, int Ng, int prec);
 void fft_plan_destroy(FftPlan *p);
-// forward r2c (sign -1) of `ngrids` in-place padded grids, unnormalised
-int fft_r2c(const FftPlan *p, void *const *grids, int ngrids, cudaStream_t s);
-// backward c2r (sign +1), unnormalised
-int fft_c2r(const FftPlan *p, void *const *grids, int ngrids, cudaStream_t s);
+// forward r2c (sign -1) of `ngrids` in-place padded grids, times scale
+int fft_r2c(const FftPlan *p, void *const *grids, int ngrids, cudaStream_t s, double scale = 1);
+// backward c2r (sign +1), times scale
+int fft_c2r(const FftPlan *p, void *const *grids, int ngrids, cudaStream_t s, double scale = 1);
 // the three passes separately (used by the fused pipeline)
 int fft_pass_k_r2c(const FftPlan *p, void *const *grids, int ngrids, cudaStream_t s);
 int fft_pass_j(const FftPlan *p, void *const *grids, int ngrids, int sign, cudaStream_t s);
-int fft_pass_i(const FftPlan *p, void *const *grids, int ngrids, int sign, cudaStream_t s);
+int fft_pass_i(const FftPlan *p, void *const *grids, int ngrids, int sign, cudaStream_t s, double scale = 1);
 
 // two-level FP32 kernels (fft2.cu) for power-of-two Ng in [4, 1024]
 bool fft2_supported(int Ng, int prec);
 int fft2_cols(int N, const void *W, void *g0, void *g1, int ngrids, int ncols, long es, long bs,
-              long nbatch, int sign, cudaStream_t s, int logC_req = -1);
+              long nbatch, int sign, cudaStream_t s, int logC_req = -1, double scale = 1);
 int fft2_k_r2c(int Ng, const void *W, const void *rtw, void *g0, void *g1, int ngrids, cudaStream_t s,
                int R_req = 0);
 // launch shape `v` of pass `which` (0 = k rows per CTA, 1 = j / 2 = i log2
@@ -104,6 +104,12 @@ int fft2_prepare();
 bool fft2_tma_supported(int Ng, int prec);
 int fft2_cols_tma(int Ng, const void *W, void *g0, void *g1, int ngrids, int sign, cudaStream_t s);
 int fft2_tma_check();
+// mixed-radix FP32 passes (fft3.cu): Ng = N1 N2 with N1, N2 <= 32 and prime
+// factors up to 13; the k pass both ways (forward r2c, backward c2r)
+bool fft3_supported(int Ng, int prec);
+int fft3_cols(int N, const void *W, void *g0, void *g1, int ngrids, int ncols, long es, long bs, long nbatch, int sign,
+              double scale, cudaStream_t s);
+int fft3_k(int Ng, const void *W, void *g0, void *g1, int ngrids, bool forward, double scale, cudaStream_t s);
 // time every valid launch shape of the three r2c passes on `grid` (one FP32
 // grid of the plan's size; its contents are transformed in place) and keep the
 // fastest in p->tune; ms[3] = the chosen shapes' times
