@@ -615,7 +615,7 @@ static fft_t *grid_new(int Ng, double L, const char *wisdom, bool host_view, boo
     if (cuda_check(cudaMalloc(&g->d_f, (size_t)g->prec * self->Ng3_pad), "grid")) return fail();
     if (cuda_check(cudaMemsetAsync(g->d_f, 0, (size_t)g->prec * self->Ng3_pad, g->stream), "grid")) return fail();
     if (fft_plan_create(&g->fft, Ng, g->prec)) return fail();
-    if (paint_tiling_create(&g->tiling, Ng)) return fail();
+    if (paint_tiling_create(&g->tiling, Ng, g->prec)) return fail();
     if (cuda_check(cudaStreamSynchronize(g->stream), "init")) return fail();
     if (!wisdom || !strcmp(wisdom, "FFTW_ESTIMATE")) {
         if (!g->quiet)

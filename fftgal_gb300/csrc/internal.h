@@ -137,7 +137,7 @@ struct PaintTiling {
     int tmax[3] = {0, 0, 0};      // largest tile extent along i, j, k
     int *d_tables = nullptr;      // device, per axis a: tile_of[Ng], then start[nt[a]+1]
     int tab_off[3] = {0, 0, 0};   // offset of axis a's tables in d_tables
-    long nkeys = 0;               // nt0*nt1*nt2 * 27
+    long nkeys = 0;               // nt0*nt1*nt2 * 27 (FP32 grids: 27 boundary classes) or * 1 (FP64)
     int cta_per_sm = 0;           // persistent FP32 tile-paint CTAs per SM (1 or 2; 0: built-in 2)
     // tiles of up to 32 x 16 x 32 cells for FP32 paints of one grid (owned;
     // null where Ng < 64): the one grid's accumulators fill the shared memory
@@ -162,7 +162,7 @@ struct PaintGridSpec {
     int accumulate = 0;           // 0: overwrite (and zero padding), 1: out += value
 };
 
-int paint_tiling_create(PaintTiling *t, int Ng);
+int paint_tiling_create(PaintTiling *t, int Ng, int prec);
 void paint_tiling_destroy(PaintTiling *t);
 void paint_scratch_free(PaintScratch *s);
 

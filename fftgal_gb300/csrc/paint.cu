@@ -99,8 +99,6 @@ constexpr int kMaxFixBits = 23;
 // records (most of 1 ms of the tile paint for a 1e8-galaxy lognormal mock at
 // Ng=1024) is skipped for moderately dense tiles
 constexpr int kBlockCountBelow = 21;
-// FP64 shared layout: dense [16][16][32]
-constexpr int kT3 = 16 * 16 * 32;
 // per-tile block counts: 4^3-cell blocks over the tile plus a 4-cell margin
 constexpr int kBlk = 4;
 __host__ __device__ constexpr int blk_dim(int a) { return a == 1 ? (16 + 8) / kBlk : (32 + 8) / kBlk; }  // 10, 6, 10
@@ -187,16 +185,26 @@ __device__ __forceinline__ void pcs_weights(float d, float w[4], float s = 1.f /
     w[3] = __fmul_rn(__fmul_rn(d2, d), s);
 }
 
+// x / 6 rounded to nearest: with r = RN(1/6) and q = RN(x r) within an ulp of x / 6,
+// RN(q + (x - 6 q) r) is the correctly rounded quotient (Markstein 1990); the
+// weights' numerators (0 .. 6, or below by roundings of 0) never make it
+// underflow.  Three operations of the FP64 pipe, which does two lanes per cycle
+// and SM.
+__device__ __forceinline__ double sixth(double x) {
+    const double r = 1.0 / 6.0;
+    const double q = __dmul_rn(x, r);
+    return __fma_rn(__fma_rn(-6.0, q, x), r, q);
+}
+
 __device__ __forceinline__ void pcs_weights(double d, double w[4]) {
     // src/fft.c:83-88 in the reference's operation order, no FMA contraction
     const double e = __dsub_rn(1.0, d);
     const double d2 = __dmul_rn(d, d);
-    w[0] = __ddiv_rn(__dmul_rn(__dmul_rn(e, e), e), 6.0);
-    w[1] = __ddiv_rn(__dadd_rn(__dmul_rn(__dsub_rn(__dmul_rn(3.0, d), 6.0), d2), 4.0), 6.0);
-    w[2] = __ddiv_rn(
-        __dadd_rn(__dmul_rn(__dadd_rn(__dmul_rn(__dadd_rn(__dmul_rn(-3.0, d), 3.0), d), 3.0), d), 1.0),
-        6.0);
-    w[3] = __ddiv_rn(__dmul_rn(d2, d), 6.0);
+    w[0] = sixth(__dmul_rn(__dmul_rn(e, e), e));
+    w[1] = sixth(__dadd_rn(__dmul_rn(__dsub_rn(__dmul_rn(3.0, d), 6.0), d2), 4.0));
+    w[2] = sixth(
+        __dadd_rn(__dmul_rn(__dadd_rn(__dmul_rn(__dadd_rn(__dmul_rn(-3.0, d), 3.0), d), 3.0), d), 1.0));
+    w[3] = sixth(__dmul_rn(d2, d));
 }
 
 // FP32 path: the grid-0 base cell b0 and the fraction as fb-bit fixed point;
@@ -238,7 +246,7 @@ template <> struct Rec<double> { struct type { double x, y, z; }; };
 template <typename P>
 __device__ __forceinline__ uint32_t paint_key_of(const P pos[3], const PaintParams &pp, uint32_t *rec = nullptr) {
     const int Ng = pp.Ng;
-    int t[3], cls[3];
+    int t[3], cls[3] = {0, 0, 0};
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         int b0;
@@ -260,26 +268,24 @@ __device__ __forceinline__ uint32_t paint_key_of(const P pos[3], const PaintPara
             t0 = pp.start[a][ta];
             te = pp.start[a][ta + 1] - t0;
         }
+        t[a] = ta;
+        if constexpr (sizeof(P) == 8) continue;  // the FP64 paint goes by the tile alone
         int rmin = b0 - t0, rmax = b0 - t0;
         for (int g = 1; g < pp.ngrids; ++g) {
             int bg;
-            if constexpr (sizeof(P) == 4) {
-                uint32_t dgq;
-                cell_g(b0, dq0, pp.ax[a].dq[g], pp.fb, Ng, bg, dgq);
-            } else {
-                P dg;
-                coord(pos[a], pp.ax[a], g, Ng, bg, dg);
-            }
+            uint32_t dgq;
+            cell_g(b0, dq0, pp.ax[a].dq[g], pp.fb, Ng, bg, dgq);
             int dl = bg - b0;  // -1, 0 or +1 after undoing a wrap
             dl -= dl > 1 ? Ng : 0;
             dl += dl < -1 ? Ng : 0;
             rmin = min(rmin, b0 - t0 + dl);
             rmax = max(rmax, b0 - t0 + dl);
         }
-        t[a] = ta;
         cls[a] = pp.nt[a] == 1 ? 0 : (rmin - 1 < 0 ? 1 : (rmax + 2 >= te ? 2 : 0));
     }
-    return (uint32_t)((((long)t[0] * pp.nt[1] + t[1]) * pp.nt[2] + t[2]) * 27 + cls[0] * 9 + cls[1] * 3 + cls[2]);
+    const long tile = ((long)t[0] * pp.nt[1] + t[1]) * pp.nt[2] + t[2];
+    if constexpr (sizeof(P) == 8) return (uint32_t)tile;
+    return (uint32_t)(tile * 27 + cls[0] * 9 + cls[1] * 3 + cls[2]);
 }
 
 template <typename P>
@@ -505,14 +511,6 @@ __device__ void tile_publish(int ncomb, uint32_t b, uint32_t cnt, uint32_t *seg_
     __syncthreads();
     ts.nseg = ncomb;
     ts.total = tot;
-}
-
-__device__ void tile_segments(const PaintParams &pp, const uint32_t *__restrict__ off, uint32_t *seg_begin,
-                              uint32_t *seg_pref, uint32_t *scan_ws, TileSegs &ts) {
-    tile_geometry(pp, blockIdx.x, ts);
-    uint32_t b, cnt;
-    const int ncomb = tile_segment(pp, off, blockIdx.x, threadIdx.x, b, cnt);
-    tile_publish(ncomb, b, cnt, seg_begin, seg_pref, scan_ws, ts);
 }
 
 // index of particle q of the flattened segment list (largest segment whose
@@ -1487,82 +1485,165 @@ paint_rot_kernel(PaintParams pp, const uint32_t *__restrict__ off, const uint4 *
     }
 }
 
-// FP64 grids: one thread per particle, FP64 shared atomics
-__global__ void __launch_bounds__(kPaintThreads)
-paint_tile_f64_kernel(PaintParams pp, const uint32_t *__restrict__ off,
-                      const Rec<double>::type *__restrict__ sorted, PaintOut po) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    double *acc = reinterpret_cast<double *>(smem_raw);  // [ngrids][kT3], dense [16][16][32]
-    __shared__ uint32_t seg_begin[kMaxSeg];
-    __shared__ uint32_t seg_pref[kMaxSeg + 1];
-    __shared__ uint32_t scan_ws[33];
-    const int Ng = pp.Ng, ngr = pp.ngrids;
-    for (int e = threadIdx.x; e < ngr * kT3; e += blockDim.x) acc[e] = 0.0;
+// FP64 grids: one warp per tile of 8 x 8 x 16 cells and grid (blockIdx.y), one
+// lane per particle of the tile.  The FP64 pipe does two lanes per cycle and SM
+// and bounds the kernel, so every operation counts: the sums cover the tile and
+// the cells its particles' stencils reach beyond it, so that no particle is
+// visited twice (the box is then added to the zeroed grid with FP64 atomics);
+// the weights' divisions by 6 take three operations; and a deposit is one fused
+// multiply-add on shared memory, without atomics.  That is safe because a warp
+// owns its box and its lanes never meet: as in paint_rot_kernel, cell (i, j, k)
+// lies at digits (i & 1, j & 3, k & 3) of a 2 x 4 x 4 block and lane l visits its
+// particle's cells at its own digits plus the step's, so the 32 lanes of a step
+// have 32 distinct digits (and the half warps 16 distinct bank pairs each).
+// 1e6 particles at Ng = 128, both grids: 2.44 ms with 512-thread CTAs that
+// pulled the neighbours' particles and added with shared FP64 atomics, whose
+// compare-and-swap loops repeat the addition for a whole warp.
+constexpr int kF64Ext[3] = {8, 8, 16};
+constexpr int kF64BJ = (8 + 4) / 4, kF64BK = (16 + 4) / 4;  // j and k blocks of the box
+constexpr int kF64Blocks = (8 + 4) / 2 * kF64BJ * kF64BK;
+// a warp deposits at most this many particles: the sorted particles are cut at
+// multiples of it, and a crowded tile's later pieces go to warps of their own
+// (blockIdx.x >= ntiles; the boxes are added atomically, so pieces may share a tile)
+constexpr uint32_t kF64Piece = 4096;
+
+// word of box cell (i, j, k)
+__device__ __forceinline__ int f64_row(int i) { return (i >> 1) * (kF64BJ * kF64BK * 32) + (i & 1) * 16; }
+__device__ __forceinline__ int f64_col(int j) { return (j >> 2) * (kF64BK * 32) + (j & 3) * 4; }
+__device__ __forceinline__ int f64_k(int k) { return (k >> 2) * 32 + (k & 3); }
+
+__device__ __forceinline__ void rotate4(double w[4], int r) {
+    const bool r1 = r & 1, r2 = r & 2;
+    const double a = r1 ? w[1] : w[0], b = r1 ? w[2] : w[1], c = r1 ? w[3] : w[2], d = r1 ? w[0] : w[3];
+    w[0] = r2 ? c : a;
+    w[1] = r2 ? d : b;
+    w[2] = r2 ? a : c;
+    w[3] = r2 ? b : d;
+}
+
+__global__ void __launch_bounds__(32, 9)
+paint_warp_f64_kernel(PaintParams pp, const uint32_t *__restrict__ off,
+                      const Rec<double>::type *__restrict__ sorted, PaintOut po, unsigned ntiles) {
+    __shared__ __align__(16) double acc[32 * kF64Blocks];
+    const int Ng = pp.Ng, g = blockIdx.y, lane = threadIdx.x;
+    unsigned tile = blockIdx.x;
+    uint32_t p0, p1;
+    if (blockIdx.x < ntiles) {
+        p0 = off[tile];
+        p1 = min(off[tile + 1], (p0 / kF64Piece + 1) * kF64Piece);
+    } else {
+        // the piece from p0: part of the tile that holds p0, unless that begins there
+        p0 = (blockIdx.x - ntiles + 1) * kF64Piece;
+        if (p0 >= off[ntiles]) return;
+        unsigned lo = 0, hi = ntiles - 1;  // the last tile with off[tile] <= p0
+        while (lo < hi) {
+            const unsigned mid = (lo + hi + 1) >> 1;
+            if (off[mid] <= p0) lo = mid;
+            else hi = mid - 1;
+        }
+        tile = lo;
+        if (off[tile] == p0) return;
+        p1 = min(off[tile + 1], p0 + kF64Piece);
+    }
+#pragma unroll 6
+    for (int e = lane; e < 32 * kF64Blocks; e += 32) acc[e] = 0.0;
     TileSegs ts;
-    tile_segments(pp, off, seg_begin, seg_pref, scan_ws, ts);
-    for (uint32_t q = threadIdx.x; q < ts.total; q += blockDim.x) {
-        const auto r = sorted[seg_index(q, seg_begin, seg_pref, ts.nseg)];
+    tile_geometry(pp, tile, ts);
+    // the box starts `low` cells below the tile: 1, or 2 where the grid's base
+    // cells can lie one below those of grid 0, which the sort went by
+    int low[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) low[a] = pp.ax[a].o[g] > pp.ax[a].o[0] ? 2 : 1;
+    const int lk = lane & 3, lb = (lane >> 2) & 3, la = lane >> 4;
+    volatile double *vacc = acc;
+    __syncwarp();
+    for (uint32_t q0 = p0; q0 < p1; q0 += 32) {
+        const bool valid = q0 + lane < p1;
+        Rec<double>::type r;
+        r.x = r.y = r.z = 0.0;
+        if (valid) r = sorted[q0 + lane];
         const double pos[3] = {r.x, r.y, r.z};
-        for (int g = 0; g < ngr; ++g) {
-            int loc[3][4];
-            double w[3][4];
+        int l[3];
+        double w[3][4];
+        bool in = valid;
 #pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                int b;
-                double d;
-                coord(pos[a], pp.ax[a], g, Ng, b, d);
-                pcs_weights(d, w[a]);
+        for (int a = 0; a < 3; ++a) {
+            int b;
+            double d;
+            coord(pos[a], pp.ax[a], g, Ng, b, d);
+            pcs_weights(d, w[a]);
+            int c = b - 1 - ts.t0[a] + low[a];
+            c += c < 0 ? Ng : 0;
+            c -= c >= Ng ? Ng : 0;
+            in = in && (unsigned)c <= (unsigned)ts.te[a];  // a particle of the tile has its first cell at 0 .. te
+            l[a] = c;
+        }
+        if (!in) {  // lanes without a particle go along with weight 0
+            l[0] = l[1] = l[2] = 0;
 #pragma unroll
-                for (int s = 0; s < 4; ++s) loc[a][s] = local_cell(b, s, Ng, ts.t0[a], ts.te[a]);
-            }
+            for (int s = 0; s < 4; ++s) w[0][s] = 0.0;
+        }
+        const int ra = (la - l[0]) & 1, rb = (lb - l[1]) & 3, rk = (lk - l[2]) & 3;
+        const int row[2] = {f64_row(l[0] + ra), f64_row(l[0] + 1 - ra)};
+        const double x[2][2] = {{ra ? w[0][1] : w[0][0], ra ? w[0][3] : w[0][2]},
+                                {ra ? w[0][0] : w[0][1], ra ? w[0][2] : w[0][3]}};
+        rotate4(w[1], rb);
+        rotate4(w[2], rk);
+        int col[4], kc[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                if (loc[0][i] < 0) continue;
+        for (int t = 0; t < 4; ++t) {
+            col[t] = f64_col(l[1] + ((rb + t) & 3));
+            kc[t] = f64_k(l[2] + ((rk + t) & 3));
+        }
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    if (loc[1][j] < 0) continue;
-                    const double wij = __dmul_rn(w[0][i], w[1][j]);
-                    double *row = acc + g * kT3 + (loc[0][i] * 16 + loc[1][j]) * 32;
+        for (int ta = 0; ta < 2; ++ta)
 #pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        if (loc[2][k] >= 0) atomicAdd(row + loc[2][k], __dmul_rn(wij, w[2][k]));
+            for (int tb = 0; tb < 4; ++tb) {
+                const double w0 = __dmul_rn(x[ta][0], w[1][tb]), w1 = __dmul_rn(x[ta][1], w[1][tb]);
+                const int rc = row[ta] + col[tb];
+#pragma unroll
+                for (int tk = 0; tk < 4; ++tk) {
+                    volatile double *p = vacc + rc + kc[tk];
+                    const double a0 = p[0], a1 = p[kF64BJ * kF64BK * 32];  // rows i and i + 2
+                    p[0] = __fma_rn(w0, w[2][tk], a0);
+                    p[kF64BJ * kF64BK * 32] = __fma_rn(w1, w[2][tk], a1);
+                    __syncwarp();
                 }
             }
-        }
     }
-    __syncthreads();
-    const bool last_k = (ts.t0[2] + ts.te[2] == Ng);
-    const int pad = last_k ? pp.Ng_pad - Ng : 0;
-    const int rowlen = ts.te[2] + pad;
-    const int ncell = ts.te[0] * ts.te[1] * rowlen;
-    for (int g = 0; g < ngr; ++g) {
-        double *out = reinterpret_cast<double *>(po.out[g]);
-        const double sc = po.scale[g];
-        const int accu = po.accumulate[g];
-        for (int e = threadIdx.x; e < ncell; e += blockDim.x) {
-            const int lk = e % rowlen, lj = (e / rowlen) % ts.te[1], li = e / (rowlen * ts.te[1]);
-            const long gi = ((long)(ts.t0[0] + li) * Ng + (ts.t0[1] + lj)) * pp.Ng_pad + ts.t0[2] + lk;
-            // padding cells: 0 x scale, like the reference's scaling of the whole grid
-            const double v = __dmul_rn(lk < ts.te[2] ? acc[g * kT3 + (li * 16 + lj) * 32 + lk] : 0.0, sc);
-            if (accu) {
-                if (lk < ts.te[2]) out[gi] = __dadd_rn(out[gi], v);
-            } else {
-                out[gi] = v;
-            }
-        }
+    __syncwarp();
+    double *out = reinterpret_cast<double *>(g ? po.out[1] : po.out[0]);
+    const double sc = g ? po.scale[1] : po.scale[0];
+    const int accu = g ? po.accumulate[1] : po.accumulate[0];
+    const bool finite = isfinite(sc);
+    for (int b = 0; b < kF64Blocks; ++b) {
+        const double v = __dmul_rn(acc[b * 32 + lane], sc);
+        const int li = b / (kF64BJ * kF64BK) * 2 + la, lj = b / kF64BK % kF64BJ * 4 + lb, lkk = b % kF64BK * 4 + lk;
+        if (!finite ? (li >= ts.te[0] || lj >= ts.te[1] || lkk >= ts.te[2]) : v == 0.0) continue;
+        const int i = (ts.t0[0] + li - (finite ? low[0] : 0) + 2 * Ng) % Ng;
+        const int j = (ts.t0[1] + lj - (finite ? low[1] : 0) + 2 * Ng) % Ng;
+        const int k = (ts.t0[2] + lkk - (finite ? low[2] : 0) + 2 * Ng) % Ng;
+        atomicAdd(out + ((long)i * Ng + j) * pp.Ng_pad + k, v);
+    }
+    // the row padding takes 0 x scale, like the reference's scaling of the whole grid
+    const int pad = blockIdx.x < ntiles && ts.t0[2] + ts.te[2] == Ng && !accu ? pp.Ng_pad - Ng : 0;
+    for (int e = lane; e < ts.te[0] * ts.te[1] * pad; e += 32) {
+        const int q = e % pad, lj = (e / pad) % ts.te[1], li = e / (pad * ts.te[1]);
+        out[((long)(ts.t0[0] + li) * Ng + ts.t0[1] + lj) * pp.Ng_pad + Ng + q] = __dmul_rn(0.0, sc);
     }
 }
 
 // ---- host side -----------------------------------------------------------------------------
 
-static int tiling_build(PaintTiling *t, int Ng, const int ext[3]) {
+static int tiling_build(PaintTiling *t, int Ng, const int ext[3], int classes) {
     std::vector<int> tab;
-    long nk = 27;
+    long nk = classes;
     for (int a = 0; a < 3; ++a) {
         int nt = (int)ceil_div(Ng, ext[a]);
-        // with more than one tile per axis every extent must be >= 5 so that a
-        // stencil reaches at most the adjacent tile and the classes are exclusive
-        while (nt > 1 && Ng / nt < 5) --nt;
+        // with more than one tile per axis and boundary classes every extent must be
+        // >= 5 so that a stencil reaches at most the adjacent tile and the classes
+        // are exclusive
+        while (classes > 1 && nt > 1 && Ng / nt < 5) --nt;
         t->tab_off[a] = (int)tab.size();
         const size_t base = tab.size();
         tab.resize(base + Ng + nt + 1);
@@ -1586,11 +1667,12 @@ static int tiling_build(PaintTiling *t, int Ng, const int ext[3]) {
     return OK;
 }
 
-int paint_tiling_create(PaintTiling *t, int Ng) {
-    FG_TRY(tiling_build(t, Ng, kTileExt));
+int paint_tiling_create(PaintTiling *t, int Ng, int prec) {
+    if (prec == 8) return tiling_build(t, Ng, kF64Ext, 1);
+    FG_TRY(tiling_build(t, Ng, kTileExt, 27));
     if (Ng >= 64) {
         t->one = new PaintTiling();
-        FG_TRY(tiling_build(t->one, Ng, kTileExt1));
+        FG_TRY(tiling_build(t->one, Ng, kTileExt1, 27));
     }
     return OK;
 }
@@ -1755,11 +1837,11 @@ int paint(const PaintTiling *t, PaintScratch *s, int grid_prec, const void *x, c
                 paint_coop_kernel<2><<<nb, T, smem, st>>>(pp, s->hist, (const uint4 *)s->sorted, po, ntiles);
         }
     } else {
-        const size_t smem = (size_t)ngrids * kT3 * sizeof(double);
-        FG_CUDA(cudaFuncSetAttribute(paint_tile_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem));
-        paint_tile_f64_kernel<<<ntiles, kPaintThreads, smem, st>>>(pp, s->hist,
-                                                                    (const Rec<double>::type *)s->sorted, po);
+        for (int g = 0; g < ngrids; ++g)
+            if (!grids[g].accumulate)
+                FG_CUDA(cudaMemsetAsync(grids[g].out, 0, sizeof(double) * (size_t)Ng * Ng * pp.Ng_pad, st));
+        paint_warp_f64_kernel<<<dim3(ntiles + (unsigned)(Np / kF64Piece), ngrids), 32, 0, st>>>(
+            pp, s->hist, (const Rec<double>::type *)s->sorted, po, ntiles);
     }
     FG_LAUNCHED(1);
     if (ev) FG_CUDA(cudaEventRecord(ev[3], st));

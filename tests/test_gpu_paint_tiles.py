@@ -1,8 +1,8 @@
-"""The tile paint of FP32 grids with Ng >= 64 (csrc/paint.cu) against the FP64
-oracle, at the grid sizes where its tiles differ: two tiles along an axis,
-extents that are odd or vary from tile to tile (144 and 175: a CTA paints tiles
-of different widths along k in turn), rows that start 16-byte aligned, 8 bytes off in
-turn, or neither (odd Ng), with catalogs that are uniform, wrapped over several
+"""The tile paints of csrc/paint.cu against the FP64 oracle: FP64 grids
+(test_paint_fp64) and FP32 grids with Ng >= 64, at the grid sizes where the tiles
+differ: two tiles along an axis, extents that are odd or vary from tile to tile
+(144 and 175: a CTA paints tiles of different widths along k in turn), rows that
+start 16-byte aligned, 8 bytes off in turn, or neither (odd Ng), with catalogs that are uniform, wrapped over several
 boxes, clumped (dense tiles) and empty, one grid with offsets and randoms and
 both interlacing grids.
 
@@ -95,3 +95,28 @@ def test_paint_both_grids(fg, oracle_lib, Ng):
     o = oracle_lib.Oracle(Ng, L)
     o.p2k(x, y, z, V)
     _close(g.exportf(), np.array(o.f), 2e-5)
+
+
+@pytest.mark.parametrize("Ng", [5, 8, 9, 18, 24, 33, 66, 90])
+@pytest.mark.parametrize("kind,offset", [("uniform", (0.0, 0.0, 0.0)), ("wrapped", (0.5, -0.3, 0.25)),
+                                         ("clump", (0.5, 0.5, 0.5)), ("empty", (0.0, 0.5, 0.0))])
+def test_paint_fp64(fg, oracle_lib, Ng, kind, offset):
+    """FP64 grids: one warp per tile of up to 8 x 8 x 16 cells, boxes that wrap,
+    tiles of more particles than one warp takes (30000 in a few cells).  A cell
+    sums up to some 1e4 terms in another order than the oracle: 1e-12 of the
+    largest cell, the FP64 grids' stated tolerance."""
+    L = 100.0
+    V = L ** 3
+    x, y, z = _catalog(kind, Ng, L)
+    g = fg.Grid(Ng, L, precision="f64", host_view="lazy")
+    cat = fg.Catalog(x, y, z, V)
+    g.p2g(cat, offset)
+    o = oracle_lib.Oracle(Ng, L)
+    o.p2g(x, y, z, V, offset)
+    if kind == "empty":
+        assert np.isnan(g.exportf()).all()
+        return
+    _close(g.exportf(), np.array(o.f), 1e-12)
+    g.p2k(cat)
+    o.p2k(x, y, z, V)
+    _close(g.exportf(), np.array(o.f), 1e-12)
