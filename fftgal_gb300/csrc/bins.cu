@@ -305,8 +305,20 @@ bin_power_kernel(BinDev d, const T *__restrict__ f, T Vinv, T Pshot,
 //   MODE 5: as 2 with the finished value binned but not written back (the
 //           fused calls under the lazy host view: 4.3 GB fewer writes at
 //           Ng = 1024).
+//
+// Mirrored modes.  A mode's k bin, wedge and Legendre weights depend on n^2 and
+// |n . los|, so modes that differ by the sign of n_i where los_i = 0 (or where
+// los has no other component) share them exactly, and likewise for n_j; where
+// only los_k = 0, (n_i, n_j) and (-n_i, -n_j) do.  The slabs then cover
+// n_i >= 0 (n_j >= 0) only: a slab element sums the powers of its NP = 4 (lines
+// of sight along an axis) or 2 (los with two components) mirrored modes, and the
+// classification, which is most of a mode's instructions, is done once for
+// them (slab_mirror; NP = 1 for other lines of sight).  Measured with their
+// finish, interlaced: Ng = 1024, los z 4.51 -> 1.94 ms (8.6 GB read: 4.4 TB/s); Ng =
+// 512 los z with ten wedges 594 -> 305 us, los (1, 1, 0) 590 -> 479 us; and with shorter
+// slabs on small grids Ng = 128 45 -> 25 us, Ng = 64 54 -> 26 us.
 constexpr int kSlabI = 16, kSlabJ = 16, kSlabK = 32, kSlabRow = 33;
-constexpr int kSlabThreads = 512;  // one warp per slab of a block
+constexpr int kSlabThreads = 512;  // one warp per slab of a block (fewer where there are few blocks)
 // blocks between folds of the FP32 sums into FP64: FFTGAL_BIN_FOLD, default 8
 static int fold_blocks() {
     static const int v = [] {
@@ -325,6 +337,27 @@ struct SlabFinish {
     float scale = 0.f;           // H^3 / 2
 };
 
+// which axes mirror, and the rows along i and j that the slabs cover
+struct SlabMirror {
+    bool fi = false, fj = false;  // n_i, n_j on their own
+    bool joint = false;           // (n_i, n_j) together
+    int NI = 0, NJ = 0;
+    __host__ __device__ int modes() const { return fi && fj ? 4 : (fi || fj || joint ? 2 : 1); }
+};
+
+static SlabMirror slab_mirror(const BinSpec &s) {
+    SlabMirror m;
+    const bool z0 = s.los[0] == 0, z1 = s.los[1] == 0, z2 = s.los[2] == 0;
+    const int nz = (z0 ? 0 : 1) + (z1 ? 0 : 1) + (z2 ? 0 : 1);
+    m.fi = z0 || nz == 1;
+    m.fj = z1 || nz == 1;
+    m.joint = z2 && !m.fi && !m.fj;
+    const int half = s.Ng / 2 + 1;
+    m.NI = m.fi || m.joint ? half : s.Ng;
+    m.NJ = m.fj ? half : s.Ng;
+    return m;
+}
+
 // The slab blocks cover k < kmain.  When the half spectrum's last k block
 // would hold only one or two columns (nh = Ng/2 + 1: the Nyquist column of
 // every even Ng that is a multiple of 32), those columns are binned mode by
@@ -336,42 +369,67 @@ __host__ __device__ __forceinline__ int slab_kmain(int nh) {
     return (nh > kSlabK && r > 0 && r <= 2) ? nh - r : nh;
 }
 
-// |delta|^2 Vinv - Pshot of element e.  MODE 2 to 5 finish it first, with the
-// phase pf * phr (MODE 2 and 5) and the window inverse wf * wr; MODE 2 and 3
-// store the finished value.
+// A mode's value and its share of the slab element: |delta|^2 without the
+// window and Vinv (MODE >= 2), |delta|^2 (MODE 1), P (MODE 0); p is the phase
+// of element e, wk the window inverse (stored with the value by MODE 2 and 3)
+struct ModeLoad {
+    float2 a, b;
+};
 template <int MODE>
-__device__ __forceinline__ float mode_power(const SlabFinish &fin, const float2 *__restrict__ f, long e, float2 pf,
-                                           float2 phr, float wf, float wr, float Vinv, float Pshot) {
+__device__ __forceinline__ ModeLoad mode_load(const SlabFinish &fin, const float2 *__restrict__ f, long e) {
+    ModeLoad m;
+    m.a = MODE == 2 || MODE == 3 ? fin.A[e] : f[e];  // these modes also write A
+    m.b = MODE == 2 || MODE == 5 ? fin.B[e] : make_float2(0.f, 0.f);
+    return m;
+}
+template <int MODE>
+__device__ __forceinline__ float mode_value(const SlabFinish &fin, const ModeLoad &m, long e, float2 p, float wk,
+                                            bool store) {
+    if (MODE == 0) return m.a.x;
+    float2 v = m.a;
     if (MODE == 2 || MODE == 5) {
-        const float2 p = cmul(pf, phr);
-        const float wk = wf * wr;
-        const float2 bv = fin.B[e], av = fin.A[e];
-        const float2 dv = cmul(bv, p);
-        const float2 v = make_float2((dv.x + av.x) * wk, (dv.y + av.y) * wk);
-        if (MODE == 2) fin.A[e] = v;
-        return (v.x * v.x + v.y * v.y) * Vinv - Pshot;
-    } else if (MODE == 3 || MODE == 4) {
-        const float wk = wf * wr;
-        const float2 av = fin.A[e];
-        const float2 v = make_float2(av.x * wk, av.y * wk);
-        if (MODE == 3) fin.A[e] = v;
-        return (v.x * v.x + v.y * v.y) * Vinv - Pshot;
-    } else if (MODE == 1) {
-        const float2 v = f[e];
-        return (v.x * v.x + v.y * v.y) * Vinv - Pshot;
-    } else {
-        return f[e].x;
+        v.x += m.b.x * p.x - m.b.y * p.y;
+        v.y += m.b.x * p.y + m.b.y * p.x;
     }
+    if ((MODE == 2 || MODE == 3) && store) fin.A[e] = make_float2(v.x * wk, v.y * wk);
+    return v.x * v.x + v.y * v.y;
+}
+// power of `count` modes whose mode_value()s sum to s
+template <int MODE>
+__device__ __forceinline__ float mode_power(float s, float count, float wk, float Vinv, float Pshot) {
+    if (MODE == 0) return s;
+    if (MODE == 1) return s * Vinv - count * Pshot;
+    return (s * wk) * wk * Vinv - count * Pshot;
 }
 
-// MINB: CTAs per SM the registers are budgeted for (3: 40 registers with a
-// few spills, 2: no spills), chosen by the CTAs per SM that the launch's
-// shared memory allows and the tuned launch shape
-template <int MODE, int MINB>
+// One mode by itself, by one thread (the columns and rows beside the slabs)
+template <int MODE>
+__device__ __forceinline__ void bin_single(const BinDev &d, const SlabFinish &fin, const float2 *__restrict__ f,
+                                           const uint32_t *thr, float *acc32, int i, int j, int k, float Vinv,
+                                           float Pshot) {
+    const int Ng = d.Ng;
+    const long e = ((long)i * Ng + j) * d.nh + k;
+    float2 p = make_float2(0.f, 0.f);
+    float wk = 0.f;
+    if (MODE == 2 || MODE == 5) p = cmul(cmul(fin.ph[Ng + j], fin.ph[2 * Ng + k]), fin.ph[i]);
+    if (MODE >= 2) wk = fin.w[j] * fin.w[k] * fin.scale * fin.w[i];
+    const float s = mode_value<MODE>(fin, mode_load<MODE>(fin, f, e), e, p, wk, true);
+    BinRun run;
+    run.add(d, thr, acc32, kval(i, Ng), kval(j, Ng), kval(k, Ng), k, mode_power<MODE>(s, 1.f, wk, Vinv, Pshot));
+    run.finish(d, acc32);
+}
+
+// MINB: CTAs per SM the registers are budgeted for, chosen by the CTAs per SM
+// that the launch's shared memory allows and the tuned launch shape.
+// nr: rows of a slab and modes of a run, 16 or, on small grids, 8 or 4, so that
+// a block makes 16 x 16 / nr slabs for as many warps (a warp takes 20 us or more
+// for 16 rows, whatever the grid; the CTA's blockDim.x / 32 warps take as many
+// slabs of a block per turn).
+template <int MODE, int NP, int MINB>
 __global__ void __launch_bounds__(kSlabThreads, MINB)
-bin_power_slab_kernel(BinDev d, const float2 *__restrict__ f, SlabFinish fin, float Vinv, float Pshot,
+bin_power_slab_kernel(BinDev d, const float2 *__restrict__ f, SlabFinish fin, SlabMirror mir, float Vinv, float Pshot,
                       const uint32_t *__restrict__ thr_g, double *__restrict__ gacc, const DevScalars *__restrict__ ds,
-                      int fold) {
+                      int fold, int nr) {
     if (ds) {
         Vinv = ds->Vinv;
         Pshot = ds->Pshot;
@@ -380,70 +438,125 @@ bin_power_slab_kernel(BinDev d, const float2 *__restrict__ f, SlabFinish fin, fl
     const int NK = d.NK, W = d.W, NQ = 4 + W;
     float *acc32 = reinterpret_cast<float *>(smem_raw);                        // [NQ][NK]
     uint32_t *thr = reinterpret_cast<uint32_t *>(acc32 + (size_t)NK * NQ);     // [NK + 2]
-    float *slabs = reinterpret_cast<float *>(thr + ((NK + 2 + 3) & ~3));        // [16][16][kSlabRow]
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    float *slabs = reinterpret_cast<float *>(thr + ((NK + 2 + 3) & ~3));        // [warps][16][kSlabRow]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5;
     float *slab = slabs + warp * kSlabJ * kSlabRow;
     for (int e = tid; e < NK * NQ; e += blockDim.x) acc32[e] = 0.f;
     for (int e = tid; e < NK + 2; e += blockDim.x) thr[e] = thr_g[e];
     __syncthreads();
-    const int Ng = d.Ng, nh = d.nh, kmain = slab_kmain(nh);
-    const int nbi = (Ng + kSlabI - 1) / kSlabI, nbj = (Ng + kSlabJ - 1) / kSlabJ, nbk = (kmain + kSlabK - 1) / kSlabK;
-    const int nblk = nbi * nbj * nbk;
+    const int Ng = d.Ng, nh = d.nh, kmain = slab_kmain(nh), NI = mir.NI, NJ = mir.NJ;
+    const int nbi = (NI + kSlabI - 1) / kSlabI, nbj = (NJ + kSlabJ - 1) / kSlabJ, nbk = (kmain + kSlabK - 1) / kSlabK;
+    const int nsub = kSlabI * (kSlabJ / nr) / nwarp;  // CTA turns per block
+    const int nblk = nbi * nbj * nbk * nsub;
+    const long si = (long)Ng * nh, sj = nh;  // element strides
     int since_fold = 0;
-    for (int blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
+    for (int turn = blockIdx.x; turn < nblk; turn += gridDim.x) {
+        const int blk = turn / nsub, sub = turn - blk * nsub;
         const int bk = blk % nbk, bj = (blk / nbk) % nbj, bi = blk / (nbk * nbj);
         const int i0 = bi * kSlabI, j0 = bj * kSlabJ, k0 = bk * kSlabK;
-        const int ci = abs(kval(min(i0 + kSlabI / 2, Ng - 1), Ng));
-        const int cj = abs(kval(min(j0 + kSlabJ / 2, Ng - 1), Ng));
+        const int ci = abs(kval(min(i0 + kSlabI / 2, NI - 1), Ng));
+        const int cj = abs(kval(min(j0 + kSlabJ / 2, NJ - 1), Ng));
         const int ck = min(k0 + kSlabK / 2, nh - 1);
         const int axis = (ck <= ci && ck <= cj) ? 2 : (cj <= ci ? 1 : 0);  // run axis
         // the warp's slab: for runs along i it fixes j and its rows are i,
         // otherwise it fixes i and its rows are j
         const bool rows_i = axis == 0;
-        const int fixed = (rows_i ? j0 : i0) + warp;
-        const int r0 = rows_i ? i0 : j0;
+        const int unit = sub * nwarp + warp;
+        const int fixed = (rows_i ? j0 : i0) + (unit & (kSlabI - 1));
+        const int r0 = (rows_i ? i0 : j0) + unit / kSlabI * nr;
+        const int nfix = rows_i ? NJ : NI, nrow = rows_i ? NI : NJ;
         const int k = k0 + lane;
-        if (fixed < Ng) {
-            float2 pfk = make_float2(0.f, 0.f);
+        if (fixed < nfix) {
+            // mirrored index along the rows (cr) and of the fixed axis (cf)
+            const bool cr = NP == 4 || (NP == 2 && (mir.joint || (rows_i ? mir.fi : mir.fj)));
+            const bool cf = NP == 4 || (NP == 2 && (mir.joint || (rows_i ? mir.fj : mir.fi)));
+            const bool has_f = fixed > 0 && 2 * fixed != Ng;
+            const int fm = fixed ? Ng - fixed : 0;
+            float2 q0 = make_float2(0.f, 0.f), q1 = q0;
             float wfk = 0.f;
             if (MODE >= 2 && k < kmain) {
-                if (MODE == 2 || MODE == 5) pfk = cmul(fin.ph[(rows_i ? Ng : 0) + fixed], fin.ph[2 * Ng + k]);
+                if (MODE == 2 || MODE == 5) {
+                    const float2 pf = fin.ph[(rows_i ? Ng : 0) + fixed], pk = fin.ph[2 * Ng + k];
+                    q0 = cmul(pf, pk);
+                    if (NP > 1) q1 = cf ? cmul(cconj(pf), pk) : q0;
+                }
                 wfk = fin.w[fixed] * fin.w[k] * fin.scale;
             }
-            // the row tables of the slab's 16 rows: lane r holds row r's, the
+            // the row tables of the slab's rows: lane r holds row r's, the
             // loop takes them by shuffle
             float2 phl = make_float2(0.f, 0.f);
             float wl = 0.f;
-            if (MODE >= 2 && lane < kSlabJ && r0 + lane < Ng) {
+            if (MODE >= 2 && lane < nr && r0 + lane < nrow) {
                 if (MODE == 2 || MODE == 5) phl = fin.ph[(rows_i ? 0 : Ng) + r0 + lane];
                 wl = fin.w[r0 + lane];
             }
-            const long estep = rows_i ? (long)Ng * nh : (long)nh;  // elements between consecutive rows
-            long e = (rows_i ? ((long)r0 * Ng + fixed) : ((long)fixed * Ng + r0)) * nh + k;
-#pragma unroll 8
-            for (int r = 0; r < kSlabJ; ++r, e += estep) {
-                float2 phr = make_float2(0.f, 0.f);
+            const long rs = rows_i ? si : sj, fs = rows_i ? sj : si;
+            const float2 *fk = f;
+            const long eF = fixed * fs + k, eG = (cf ? fm : fixed) * fs + k;
+            // unrolled for 8 or 16 loads in flight, as far as the registers go
+            constexpr int UNR = MINB >= 3 ? (NP == 1 ? 8 : 4 / NP) : (NP == 1 ? 8 : 8 / NP);
+#pragma unroll UNR
+            for (int r = 0; r < nr; ++r) {
+                float2 pr = make_float2(0.f, 0.f);
                 float wr = 0.f;
                 if (MODE == 2 || MODE == 5) {
-                    phr.x = __shfl_sync(0xffffffffu, phl.x, r);
-                    phr.y = __shfl_sync(0xffffffffu, phl.y, r);
+                    pr.x = __shfl_sync(0xffffffffu, phl.x, r);
+                    pr.y = __shfl_sync(0xffffffffu, phl.y, r);
                 }
                 if (MODE >= 2) wr = __shfl_sync(0xffffffffu, wl, r);
                 float pv = 0.f;
-                if (r0 + r < Ng && k < kmain) pv = mode_power<MODE>(fin, f, e, pfk, phr, wfk, wr, Vinv, Pshot);
+                const int x = r0 + r;
+                if (x < nrow && k < kmain) {
+                    const float wk = wfk * wr;
+                    const long e0 = x * rs + eF;
+                    if (NP == 1) {
+                        const float s = mode_value<MODE>(fin, mode_load<MODE>(fin, fk, e0), e0, cmul(q0, pr), wk, true);
+                        pv = mode_power<MODE>(s, 1.f, wk, Vinv, Pshot);
+                    } else {
+                        const bool has_r = x > 0 && 2 * x != Ng;
+                        const long xm = x ? Ng - x : 0;
+                        const float2 pc = cconj(pr);
+                        if (NP == 2) {
+                            // one partner; jointly mirrored modes need both indices off the Nyquist
+                            // row and n_i off 0
+                            bool has = cr ? has_r : has_f;
+                            if (mir.joint)
+                                has = rows_i ? has_r && 2 * fixed != Ng : has_f && 2 * x != Ng;
+                            const long e1 = has ? (cr ? xm : x) * rs + eG : e0;
+                            const ModeLoad m0 = mode_load<MODE>(fin, fk, e0), m1 = mode_load<MODE>(fin, fk, e1);
+                            float s = mode_value<MODE>(fin, m0, e0, cmul(q0, pr), wk, true);
+                            const float t = mode_value<MODE>(fin, m1, e1, cmul(q1, cr ? pc : pr), wk, has);
+                            s += has ? t : 0.f;
+                            pv = mode_power<MODE>(s, has ? 2.f : 1.f, wk, Vinv, Pshot);
+                        } else {
+                            const long e1 = has_r ? xm * rs + eF : e0, e2 = has_f ? x * rs + eG : e0;
+                            const long e3 = has_r && has_f ? xm * rs + eG : e0;
+                            const ModeLoad m0 = mode_load<MODE>(fin, fk, e0), m1 = mode_load<MODE>(fin, fk, e1);
+                            const ModeLoad m2 = mode_load<MODE>(fin, fk, e2), m3 = mode_load<MODE>(fin, fk, e3);
+                            float s = mode_value<MODE>(fin, m0, e0, cmul(q0, pr), wk, true);
+                            const float t1 = mode_value<MODE>(fin, m1, e1, cmul(q0, pc), wk, has_r);
+                            const float t2 = mode_value<MODE>(fin, m2, e2, cmul(q1, pr), wk, has_f);
+                            const float t3 = mode_value<MODE>(fin, m3, e3, cmul(q1, pc), wk, has_r && has_f);
+                            s += has_r ? t1 : 0.f;
+                            s += has_f ? t2 : 0.f;
+                            s += has_r && has_f ? t3 : 0.f;
+                            pv = mode_power<MODE>(s, (has_r ? 2.f : 1.f) * (has_f ? 2.f : 1.f), wk, Vinv, Pshot);
+                        }
+                    }
+                }
                 slab[r * kSlabRow + lane] = pv;
             }
         }
         __syncwarp();
-        if (fixed < Ng) {
-            // runs along k: lane = (row, half of the 32 k); else lane = k
+        if (fixed < nfix) {
+            // runs along k: lane = (row, stretch of nr of the 32 k); else lane = k
             if (axis == 2) {
-                const int r = lane & 15, c = 16 * (lane >> 4), rr = r0 + r, kc = k0 + c;
-                const int n = rr < Ng ? min(16, kmain - kc) : 0;
+                const int r = lane & (nr - 1), c = lane - r, rr = r0 + r, kc = k0 + c;
+                const int n = rr < nrow ? min(nr, kmain - kc) : 0;
                 bin_run<2>(d, thr, acc32, fixed, rr, kc, n, slab + r * kSlabRow + c, 1);
             } else {
                 const int kc = k0 + lane;
-                const int n = kc < kmain ? min(16, Ng - r0) : 0;
+                const int n = kc < kmain ? min(nr, nrow - r0) : 0;
                 if (axis == 1)
                     bin_run<1>(d, thr, acc32, fixed, r0, kc, n, slab + lane, kSlabRow);
                 else
@@ -458,32 +571,22 @@ bin_power_slab_kernel(BinDev d, const float2 *__restrict__ f, SlabFinish fin, fl
             __syncthreads();
         }
     }
-    // the columns k >= kmain, one mode per thread (consecutive threads take
-    // consecutive j; the finish takes the phase and window products in the
-    // order of the blocks that run along i)
+    // beside the slabs, one mode per thread (consecutive threads take consecutive
+    // k and j): the columns k >= kmain, and, where (n_i, n_j) mirror together, the
+    // modes (-n_i, Ng/2) whose partner's n_j = -Ng/2 keeps its sign
+    const long step = (long)gridDim.x * blockDim.x, first = (long)blockIdx.x * blockDim.x + tid;
     if (kmain < nh) {
         const int ncol = nh - kmain;
-        const long nplane = (long)ncol * Ng * Ng;
-        for (long m = (long)blockIdx.x * blockDim.x + tid; m < nplane; m += (long)gridDim.x * blockDim.x) {
-            const int kc = kmain + (int)(m % ncol);
+        for (long m = first; m < (long)ncol * Ng * Ng; m += step) {
             const long ij = m / ncol;
-            const int j = (int)(ij % Ng), i = (int)(ij / Ng);
-            const long e = ((long)i * Ng + j) * nh + kc;
-            float2 pf = make_float2(0.f, 0.f), phr = make_float2(0.f, 0.f);
-            float wf = 0.f, wr = 0.f;
-            if (MODE == 2 || MODE == 5) {
-                pf = cmul(fin.ph[Ng + j], fin.ph[2 * Ng + kc]);
-                phr = fin.ph[i];
-            }
-            if (MODE >= 2) {
-                wf = fin.w[j] * fin.w[kc] * fin.scale;
-                wr = fin.w[i];
-            }
-            const float pv = mode_power<MODE>(fin, f, e, pf, phr, wf, wr, Vinv, Pshot);
-            BinRun run;
-            run.add(d, thr, acc32, kval(i, Ng), kval(j, Ng), kval(kc, Ng), kc, pv);
-            run.finish(d, acc32);
+            bin_single<MODE>(d, fin, f, thr, acc32, (int)(ij / Ng), (int)(ij % Ng), kmain + (int)(m % ncol), Vinv,
+                             Pshot);
         }
+    }
+    if (NP == 2 && mir.joint && Ng % 2 == 0) {
+        for (long m = first; m < (long)(Ng / 2 - 1) * kmain; m += step)
+            bin_single<MODE>(d, fin, f, thr, acc32, Ng / 2 + 1 + (int)(m / kmain), Ng / 2, (int)(m % kmain), Vinv,
+                             Pshot);
     }
     __syncthreads();
     for (int e = tid; e < NK * NQ; e += blockDim.x) {
@@ -495,9 +598,9 @@ bin_power_slab_kernel(BinDev d, const float2 *__restrict__ f, SlabFinish fin, fl
     }
 }
 
-static size_t slab_smem(int NK, int NQ) {
+static size_t slab_smem(int NK, int NQ, int warps = kSlabThreads / 32) {
     return sizeof(float) * (size_t)NK * NQ + sizeof(uint32_t) * (size_t)((NK + 2 + 3) & ~3) +
-           sizeof(float) * (kSlabThreads / 32) * kSlabJ * kSlabRow;
+           sizeof(float) * warps * kSlabJ * kSlabRow;
 }
 
 static int bin_launch(BinGeometry *g, const void *f, int prec, int mode, double Vinv, double Pshot, cudaStream_t st,
@@ -535,17 +638,35 @@ static int bin_launch(BinGeometry *g, const void *f, int prec, int mode, double 
     const BinSpec &s = g->spec;
     const BinDev d = make_dev(s);
     const int NK = s.NK, W = s.Nmu + 1, NQ = 4 + W;
-    const size_t smem = prec == 4 ? slab_smem(NK, NQ) : (size_t)NK * NQ * 8 + sizeof(uint32_t) * (NK + 2);
+    size_t smem = prec == 4 ? slab_smem(NK, NQ) : (size_t)NK * NQ * 8 + sizeof(uint32_t) * (NK + 2);
     if (smem > 220 * 1024)
         return set_error(ERR_UNSUPPORTED, "binning: %d k bins x %d wedges exceed shared memory", NK, s.Nmu);
     FG_CUDA(cudaMemsetAsync(g->d_acc, 0, sizeof(double) * g->acc_len, st));
     if (prec == 4) {
+        const SlabMirror mir = slab_mirror(s);
+        const int np = mir.modes();
+        // small grids: shorter slabs until there are 16 warps' worth per SM, and
+        // smaller CTAs until there are two per SM
+        const long blocks = ceil_div(mir.NI, kSlabI) * ceil_div(mir.NJ, kSlabJ) *
+                            ceil_div(slab_kmain(s.Ng / 2 + 1), kSlabK);
+        int nr = kSlabJ;
+        while (nr > 4 && blocks * kSlabI * (kSlabJ / nr) < 16L * num_sms()) nr /= 2;
+        const long units = blocks * kSlabI * (kSlabJ / nr);
+        int warps = kSlabThreads / 32;
+        while (warps > 4 && units / warps < 2L * num_sms()) warps /= 2;
+        smem = slab_smem(NK, NQ, warps);
         int per_sm = (int)((224 * 1024) / (smem + 1024));
-        per_sm = per_sm < 1 ? 1 : (per_sm > 3 ? 3 : per_sm);
+        // three CTAs per SM hide the loads best, except where four mirrored modes of
+        // two grids want 16 loads in flight and the grid is large: two CTAs without
+        // spills (interlaced, los along z: Ng = 1024 1.94 against 2.27 ms, 512 305 against
+        // 348 us, 384 158 against 180, but 256 84 against 76, 128 28.7 against 24.6; two
+        // mirrored modes at 512 524 against 479 us)
+        const bool two = np == 4 && (mode == 2 || mode == 5) && units >= 64L * num_sms();
+        per_sm = per_sm < 1 ? 1 : (per_sm > (two ? 2 : 3) ? (two ? 2 : 3) : per_sm);
         if (g->cta_per_sm > 0 && g->cta_per_sm < per_sm) per_sm = g->cta_per_sm;  // tuned shape
-        const long nblk = ceil_div(s.Ng, kSlabI) * ceil_div(s.Ng, kSlabJ) * ceil_div(slab_kmain(s.Ng / 2 + 1), kSlabK);
+        const long nturn = units / warps;
         long nb = (long)num_sms() * per_sm;
-        if (nb > nblk) nb = nblk;
+        if (nb > nturn) nb = nturn;
         SlabFinish sf;
         if (fin) {
             sf.A = static_cast<float2 *>(fin->A);
@@ -555,12 +676,22 @@ static int bin_launch(BinGeometry *g, const void *f, int prec, int mode, double 
             sf.scale = (float)fin->scale;
         }
         const float2 *fv = static_cast<const float2 *>(mode >= 2 ? fin->A : f);
-#define FG_SLAB_LAUNCH2(M, B)                                                                                \
+#define FG_SLAB_LAUNCH3(M, N, B)                                                                             \
     do {                                                                                                    \
-        FG_CUDA(cudaFuncSetAttribute(bin_power_slab_kernel<M, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                     (int)smem));                                                           \
-        bin_power_slab_kernel<M, B><<<(unsigned)nb, kSlabThreads, smem, st>>>(                              \
-            d, fv, sf, (float)Vinv, (float)Pshot, g->d_thr, g->d_acc, ds, g->fold > 0 ? g->fold : fold_blocks()); \
+        FG_CUDA(cudaFuncSetAttribute(bin_power_slab_kernel<M, N, B>,                                         \
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));               \
+        bin_power_slab_kernel<M, N, B><<<(unsigned)nb, 32 * warps, smem, st>>>(                              \
+            d, fv, sf, mir, (float)Vinv, (float)Pshot, g->d_thr, g->d_acc, ds,                               \
+            g->fold > 0 ? g->fold : fold_blocks(), nr);                                                      \
+    } while (0)
+#define FG_SLAB_LAUNCH2(M, B)            \
+    do {                                 \
+        if (np == 4)                     \
+            FG_SLAB_LAUNCH3(M, 4, B);    \
+        else if (np == 2)                \
+            FG_SLAB_LAUNCH3(M, 2, B);    \
+        else                             \
+            FG_SLAB_LAUNCH3(M, 1, B);    \
     } while (0)
 #define FG_SLAB_LAUNCH(M)             \
     do {                              \
@@ -581,6 +712,7 @@ static int bin_launch(BinGeometry *g, const void *f, int prec, int mode, double 
             FG_SLAB_LAUNCH(4);
         else
             FG_SLAB_LAUNCH(5);
+#undef FG_SLAB_LAUNCH3
 #undef FG_SLAB_LAUNCH2
 #undef FG_SLAB_LAUNCH
     } else {
