@@ -23,6 +23,7 @@
 
 #include <math.h>
 #include <stdlib.h>
+#include <atomic>
 #include <mutex>
 
 namespace fg {
@@ -768,7 +769,12 @@ bool fft2_tma_supported(int Ng, int prec) {
     return on && prec == 4 && (Ng == 512 || Ng == 1024);
 }
 
+// set by the first TMA pass (or its capture): until then no flag can be up, and
+// the check's blocking copy (10 us or more of a small call) is left out
+static std::atomic<bool> g_tma_used{false};
+
 int fft2_cols_tma(int Ng, const void *W, void *g0, void *g1, int ngrids, int sign, cudaStream_t s) {
+    g_tma_used.store(true);
     FG_TRY(ensure_w32());
     if (!fft2_tma_supported(Ng, 4)) return set_error(ERR_UNSUPPORTED, "TMA i pass: Ng=%d", Ng);
     const int nh = Ng / 2 + 1, Ng_pad = 2 * nh;
@@ -804,6 +810,7 @@ int fft2_cols_tma(int Ng, const void *W, void *g0, void *g1, int ngrids, int sig
 }
 
 int fft2_tma_check() {
+    if (!g_tma_used.load()) return OK;
     int v = 0;
     FG_CUDA(cudaMemcpyFromSymbol(&v, g_tma_err, sizeof(int)));
     if (v) {

@@ -122,7 +122,7 @@ struct PaintParams {
     float los[3], aHinv;
     int Ng, Ng_pad, ngrids;
     int fb;                  // FP32 path: fraction bits of the packed cell coordinate
-    int nt[3];
+    int nt[3], tmax[3];      // tiles per axis, and their largest extents
     const int *tile_of[3];   // [Ng] per axis
     int tshift[3];           // log2 of the tile extent when every tile of the axis has it, else -1
     const int *start[3];     // [nt + 1] per axis
@@ -300,7 +300,33 @@ __global__ void paint_key_kernel(const P *__restrict__ x, const P *__restrict__ 
     }
 }
 
+// Few keys (small grids): thousands of particles share a key, and atomics on one
+// address come one after another (1e6 particles, Ng = 128, 3456 keys: 35 us, their
+// 12 bytes per particle taking 2 us).  A CTA then counts in shared memory and
+// adds its nonzero counts.  (Ranking chunks of 2048 particles in shared memory for
+// the scatter as well was slower there: 51 against 37 us, Ng = 64 27 against 16.)
+constexpr long kFewKeys = 8192;
+template <typename P>
+__global__ void __launch_bounds__(256)
+paint_key_few_kernel(const P *__restrict__ x, const P *__restrict__ y, const P *__restrict__ z, long Np,
+                     PaintParams pp, uint32_t *__restrict__ hist, int nkeys, const DevScalars *__restrict__ ds) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    uint32_t *h = reinterpret_cast<uint32_t *>(smem_raw);  // [nkeys]
+    if (ds) Np = ds->Np;
+    for (int e = threadIdx.x; e < nkeys; e += blockDim.x) h[e] = 0u;
+    __syncthreads();
+    for (long p = blockIdx.x * (long)blockDim.x + threadIdx.x; p < Np; p += (long)gridDim.x * blockDim.x) {
+        P pos[3] = {x[p], y[p], z[p]};
+        rsd_displace(pp, p, pos);
+        atomicAdd(&h[paint_key_of<P>(pos, pp)], 1u);
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < nkeys; e += blockDim.x)
+        if (h[e]) atomicAdd(&hist[e], h[e]);
+}
+
 // ---- 2. exclusive scan of the histogram (in place, n + 1 entries) ------------------
+// The offsets are written to a second array too: the scatter's cursors.
 
 constexpr int kScanThreads = 1024;
 constexpr int kScanPer = 4;
@@ -360,7 +386,8 @@ __global__ void scan_top(uint32_t *bsum, long nb) {
     }
 }
 
-__global__ void scan_apply(uint32_t *__restrict__ a, long n, const uint32_t *__restrict__ bsum) {
+__global__ void scan_apply(uint32_t *__restrict__ a, uint32_t *__restrict__ cursor, long n,
+                           const uint32_t *__restrict__ bsum) {
     __shared__ uint32_t ws[32];
     __shared__ uint32_t tot;
     const long base = (long)blockIdx.x * kScanBlock + threadIdx.x * kScanPer;
@@ -374,21 +401,68 @@ __global__ void scan_apply(uint32_t *__restrict__ a, long n, const uint32_t *__r
     uint32_t e = block_exclusive_scan(s, ws, &tot) + bsum[blockIdx.x];
 #pragma unroll
     for (int i = 0; i < kScanPer; ++i) {
-        if (base + i < n) a[base + i] = e;
+        if (base + i < n) a[base + i] = cursor[base + i] = e;
         e += v[i];
     }
 }
 
-static int exclusive_scan(uint32_t *a, long n, uint32_t *bsum, cudaStream_t st) {
+// short arrays: one CTA runs through them in one launch
+constexpr long kScanOne = 4L * kScanBlock;
+__global__ void __launch_bounds__(kScanThreads)
+scan_one(uint32_t *__restrict__ a, uint32_t *__restrict__ cursor, int n) {
+    __shared__ uint32_t ws[32];
+    __shared__ uint32_t tot;
+    uint32_t carry = 0;
+    for (int c0 = 0; c0 < n; c0 += kScanBlock) {
+        const int base = c0 + threadIdx.x * kScanPer;
+        uint32_t v[kScanPer], s = 0;
+#pragma unroll
+        for (int i = 0; i < kScanPer; ++i) {
+            v[i] = base + i < n ? a[base + i] : 0;
+            s += v[i];
+        }
+        uint32_t e = carry + block_exclusive_scan(s, ws, &tot);
+        carry += tot;
+#pragma unroll
+        for (int i = 0; i < kScanPer; ++i) {
+            if (base + i < n) a[base + i] = cursor[base + i] = e;
+            e += v[i];
+        }
+        __syncthreads();  // tot is rewritten by the next stretch
+    }
+}
+
+static int exclusive_scan(uint32_t *a, uint32_t *cursor, long n, uint32_t *bsum, cudaStream_t st) {
+    if (n <= kScanOne) {
+        scan_one<<<1, kScanThreads, 0, st>>>(a, cursor, (int)n);
+        FG_LAUNCHED(1);
+        return OK;
+    }
     const long nb = ceil_div(n, kScanBlock);
     scan_block_sums<<<(unsigned)nb, kScanThreads, 0, st>>>(a, n, bsum);
     scan_top<<<1, kScanThreads, 0, st>>>(bsum, nb);
-    scan_apply<<<(unsigned)nb, kScanThreads, 0, st>>>(a, n, bsum);
+    scan_apply<<<(unsigned)nb, kScanThreads, 0, st>>>(a, cursor, n, bsum);
     FG_LAUNCHED(3);
     return OK;
 }
 
 // ---- 3. scatter into key order ------------------------------------------------------
+
+// the record of a displaced particle, and its key
+template <typename P>
+__device__ __forceinline__ uint32_t paint_record(const P pos[3], const PaintParams &pp, typename Rec<P>::type &r) {
+    if constexpr (sizeof(P) == 4) {
+        uint32_t w[3];
+        const uint32_t k = paint_key_of<P>(pos, pp, w);
+        r = make_uint4(w[0], w[1], w[2], 0u);
+        return k;
+    } else {
+        r.x = pos[0];
+        r.y = pos[1];
+        r.z = pos[2];
+        return paint_key_of<P>(pos, pp);
+    }
+}
 
 template <typename P>
 __global__ void paint_scatter_kernel(const P *__restrict__ x, const P *__restrict__ y,
@@ -401,17 +475,7 @@ __global__ void paint_scatter_kernel(const P *__restrict__ x, const P *__restric
         P pos[3] = {x[p], y[p], z[p]};
         rsd_displace(pp, p, pos);
         typename Rec<P>::type r;
-        uint32_t k;
-        if constexpr (sizeof(P) == 4) {
-            uint32_t w[3];
-            k = paint_key_of<P>(pos, pp, w);
-            r = make_uint4(w[0], w[1], w[2], 0u);
-        } else {
-            k = paint_key_of<P>(pos, pp);
-            r.x = pos[0];
-            r.y = pos[1];
-            r.z = pos[2];
-        }
+        const uint32_t k = paint_record<P>(pos, pp, r);
         sorted[atomicAdd(&cursor[k], 1u)] = r;
     }
 }
@@ -643,13 +707,13 @@ __device__ __forceinline__ int tile_fixbits(uint32_t total, const uint4 *__restr
     const int fixbits = fix_bits_for(total);
     if (fixbits >= kBlockCountBelow) return fixbits;
     const int Ng = pp.Ng, fb = pp.fb, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nwarp = kPaintThreads / 32;
+    const int nwarp = (int)blockDim.x / 32;
     int nb[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) nb[a] = cyc[a] ? (Ng + kBlk - 1) / kBlk : blk_dim(a);
-    for (int e = tid; e < kBlkN; e += kPaintThreads) blk[e] = 0u;
+    for (int e = tid; e < kBlkN; e += blockDim.x) blk[e] = 0u;
     __syncthreads();
-    for (uint32_t q = tid; q < total; q += kPaintThreads) {
+    for (uint32_t q = tid; q < total; q += blockDim.x) {
         const uint4 r = sorted[index(q)];
         const uint32_t rw[3] = {r.x, r.y, r.z};
         int bidx = 0;
@@ -676,7 +740,7 @@ __device__ __forceinline__ int tile_fixbits(uint32_t total, const uint4 *__restr
     // periodic axis): the largest 3x3x3 block sum bounds every cell's
     // contributor count.  Separable window sums along k, j, i.
     const int D1 = blk_dim(1), D2 = blk_dim(2);
-    for (int e = tid; e < kBlkN; e += kPaintThreads) {
+    for (int e = tid; e < kBlkN; e += blockDim.x) {
         const int k = e % D2, j = (e / D2) % D1, i = e / (D2 * D1);
         uint32_t v = 0;
         const bool in = i < nb[0] && j < nb[1] && k < nb[2] && (cyc[2] || k + 2 < nb[2]);
@@ -685,7 +749,7 @@ __device__ __forceinline__ int tile_fixbits(uint32_t total, const uint4 *__restr
         tmp[e] = v;
     }
     __syncthreads();
-    for (int e = tid; e < kBlkN; e += kPaintThreads) {
+    for (int e = tid; e < kBlkN; e += blockDim.x) {
         const int k = e % D2, j = (e / D2) % D1, i = e / (D2 * D1);
         uint32_t v = 0;
         const bool in = i < nb[0] && j < nb[1] && k < nb[2] && (cyc[1] || j + 2 < nb[1]);
@@ -695,7 +759,7 @@ __device__ __forceinline__ int tile_fixbits(uint32_t total, const uint4 *__restr
     }
     __syncthreads();
     uint32_t mx = 0;
-    for (int e = tid; e < kBlkN; e += kPaintThreads) {
+    for (int e = tid; e < kBlkN; e += blockDim.x) {
         const int k = e % D2, j = (e / D2) % D1, i = e / (D2 * D1);
         const bool in = i < nb[0] && j < nb[1] && k < nb[2] && (cyc[0] || i + 2 < nb[0]);
         if (in) {
@@ -1207,7 +1271,11 @@ __device__ __forceinline__ void rot_deposit_wide(unsigned long long *acc, const 
 // CTAs grid 1 of the same tiles, from one sort keyed for both grids.  The
 // offsets of the next tile's segments are loaded before the deposits and its
 // first records before the write-out, so their latencies hide behind them.
-__global__ void __launch_bounds__(kPaintThreads, 2)
+// T threads: 512, two CTAs per SM, or, where there are no more tiles (times
+// grids) than SMs, one CTA of 1024 (two grids of Ng = 96, 54 tiles, 3e5 particles:
+// 38 us against 45; of Ng = 64, 16 tiles, 4e4 particles: 20 against 22).
+template <int T>
+__global__ void __launch_bounds__(T, 1024 / T)
 paint_rot_kernel(PaintParams pp, const uint32_t *__restrict__ off, const uint4 *__restrict__ sorted, PaintOut po,
                  unsigned ntiles, int split) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1220,7 +1288,7 @@ paint_rot_kernel(PaintParams pp, const uint32_t *__restrict__ off, const uint4 *
     __shared__ int geo[6];         // t0, te of the tile
     __shared__ uint32_t first[2];  // the next tile's own particles: first record, count
     const int Ng = pp.Ng, fb = pp.fb, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    constexpr int nwarp = kPaintThreads / 32;
+    constexpr int nwarp = T / 32;
     const int g = split ? (int)(blockIdx.x & 1) : 0;
     const int delta[3] = {g ? pp.ax[0].dq[1] : pp.ax[0].dq[0], g ? pp.ax[1].dq[1] : pp.ax[1].dq[0],
                           g ? pp.ax[2].dq[1] : pp.ax[2].dq[0]};
@@ -1232,7 +1300,7 @@ paint_rot_kernel(PaintParams pp, const uint32_t *__restrict__ off, const uint4 *
     const unsigned ncta = split ? gridDim.x >> 1 : gridDim.x;
     unsigned tile = cta;
     if (tile >= ntiles) return;
-    for (int e = tid; e < (int)(kRotAccBytes / 16); e += kPaintThreads)
+    for (int e = tid; e < (int)(kRotAccBytes / 16); e += T)
         reinterpret_cast<uint4 *>(smem_raw)[e] = make_uint4(0, 0, 0, 0);
     // the segments of a tile, one per thread of the first four warps, and its
     // geometry, loaded into registers that nothing reads until publish() ...
@@ -1355,9 +1423,9 @@ paint_rot_kernel(PaintParams pp, const uint32_t *__restrict__ off, const uint4 *
         if (!wide) {
             const float s6k = (1.f / 6.f) * __int_as_float((127 + fixbits - 85) << 23);  // 2^(s - 85) / 6
             if ((uint32_t)tid >= own && (uint32_t)tid < total) rec = sorted[index((uint32_t)tid)];
-            for (uint32_t q = tid; q < total; q += kPaintThreads) {
+            for (uint32_t q = tid; q < total; q += T) {
                 const uint4 r = rec;
-                if (q + kPaintThreads < total) rec = sorted[index(q + kPaintThreads)];  // in flight during the deposit
+                if (q + T < total) rec = sorted[index(q + T)];  // in flight during the deposit
                 rot_deposit(acc, r, Ng, fb, rt, rl, delta, inv, s6k, lane);
             }
             if (tid == 0) {
@@ -1377,7 +1445,7 @@ paint_rot_kernel(PaintParams pp, const uint32_t *__restrict__ off, const uint4 *
                                           // scales the whole padded grid (src/fft.c:127-129)
             // shift, extent and padding are even and the rows 16-byte aligned up to their shift
             const bool pairs = vec && !accu && ((rt.sh0 | te2 | rowlen) & 1) == 0;
-            static_assert(nwarp == 16, "a warp's block rows are 8 rows apart, with one j");
+            static_assert(nwarp % 4 == 0, "a warp's block rows are nwarp / 2 rows apart, with one j");
             const int r = lane & 7, kq = lane >> 3, hi = r >> 2;
             const int j = 4 * (warp & 3) + (r & 3), sh = (r & 1) ? rt.sh1 : rt.sh0;
             const int k = 4 * (kq + 4 * hi) - sh;  // after the exchange
@@ -1413,7 +1481,8 @@ paint_rot_kernel(PaintParams pp, const uint32_t *__restrict__ off, const uint4 *
                     }
                 }
             };
-            for (int m = 0; m < 4; ++m, i += 8, src += nwarp * kRotKB * 8, o += 8 * istride) {
+            // (rows that no tile has are never read: they need no clearing)
+            for (; i < pp.tmax[0]; i += nwarp / 2, src += nwarp * kRotKB * 8, o += nwarp / 2 * istride) {
                 float4 u = take(src), v = take(src + 4 * 8);
                 const float4 snd = hi ? u : v;
                 float4 rcv;
@@ -1453,10 +1522,10 @@ paint_rot_kernel(PaintParams pp, const uint32_t *__restrict__ off, const uint4 *
             for (int h = 0; h < te0; h += 16) {
                 const int rows = min(16, te0 - h);
                 __syncthreads();
-                for (int e = tid; e < (int)(kRotAccBytes / 16); e += kPaintThreads)
+                for (int e = tid; e < (int)(kRotAccBytes / 16); e += T)
                     reinterpret_cast<uint4 *>(smem_raw)[e] = make_uint4(0, 0, 0, 0);
                 __syncthreads();
-                for (uint32_t q = tid; q < total; q += kPaintThreads)
+                for (uint32_t q = tid; q < total; q += T)
                     rot_deposit_wide(acc64, sorted[index(q)], Ng, fb, rt, h, rows, delta, inv, kscale);
                 __syncthreads();
                 for (int b = warp; b < 8 * 4 * kRotKB; b += nwarp) {
@@ -1476,7 +1545,7 @@ paint_rot_kernel(PaintParams pp, const uint32_t *__restrict__ off, const uint4 *
             }
             __syncthreads();
             if ((uint32_t)tid < first[1]) rec = sorted[first[0] + tid];
-            for (int e = tid; e < (int)(kRotAccBytes / 16); e += kPaintThreads)
+            for (int e = tid; e < (int)(kRotAccBytes / 16); e += T)
                 reinterpret_cast<uint4 *>(smem_raw)[e] = make_uint4(0, 0, 0, 0);
         }
         if (next >= ntiles) break;
@@ -1760,6 +1829,7 @@ int paint(const PaintTiling *t, PaintScratch *s, int grid_prec, const void *x, c
     if (grid_prec == 4 && pp.fb < 16) return set_error(ERR_UNSUPPORTED, "FP32 paint: Ng=%d too large", Ng);
     for (int a = 0; a < 3; ++a) {
         pp.nt[a] = t->nt[a];
+        pp.tmax[a] = t->tmax[a];
         pp.tile_of[a] = t->d_tables + t->tab_off[a];
         {
             const int ext = Ng / t->nt[a];
@@ -1789,18 +1859,28 @@ int paint(const PaintTiling *t, PaintScratch *s, int grid_prec, const void *x, c
     FG_CUDA(cudaMemsetAsync(s->hist, 0, sizeof(uint32_t) * (t->nkeys + 1), st));
     const int nsm = num_sms();
     const unsigned gp = (unsigned)(Np > 0 ? (ceil_div(Np, 256) < 32L * nsm ? ceil_div(Np, 256) : 32L * nsm) : 1);
+    // few keys: counted in shared memory, two particles or more per thread
+    const bool few = t->nkeys <= kFewKeys;
+    const size_t ksm = sizeof(uint32_t) * (size_t)t->nkeys;
+    const unsigned gf = (unsigned)(ceil_div(Np, 512) < 4L * nsm ? ceil_div(Np, 512) : 4L * nsm);
+#define FG_KEY_LAUNCH(P, D)                                                                                      \
+    do {                                                                                                        \
+        if (few)                                                                                                \
+            paint_key_few_kernel<P><<<gf, 256, ksm, st>>>((const P *)x, (const P *)y, (const P *)z, Np, pp,      \
+                                                          s->hist, (int)t->nkeys, D);                           \
+        else                                                                                                    \
+            paint_key_kernel<P><<<gp, 256, 0, st>>>((const P *)x, (const P *)y, (const P *)z, Np, pp, s->hist, D); \
+    } while (0)
     if (Np > 0) {
         if (pos_prec == 4)
-            paint_key_kernel<float><<<gp, 256, 0, st>>>((const float *)x, (const float *)y, (const float *)z, Np,
-                                                       pp, s->hist, ds);
+            FG_KEY_LAUNCH(float, ds);
         else
-            paint_key_kernel<double><<<gp, 256, 0, st>>>((const double *)x, (const double *)y, (const double *)z,
-                                                        Np, pp, s->hist, nullptr);
+            FG_KEY_LAUNCH(double, nullptr);
         FG_LAUNCHED(1);
     }
+#undef FG_KEY_LAUNCH
     if (ev) FG_CUDA(cudaEventRecord(ev[0], st));
-    FG_TRY(exclusive_scan(s->hist, t->nkeys + 1, s->scan_tmp, st));
-    FG_CUDA(cudaMemcpyAsync(s->cursor, s->hist, sizeof(uint32_t) * (t->nkeys + 1), cudaMemcpyDeviceToDevice, st));
+    FG_TRY(exclusive_scan(s->hist, s->cursor, t->nkeys + 1, s->scan_tmp, st));
     if (ev) FG_CUDA(cudaEventRecord(ev[1], st));
     if (Np > 0) {
         if (pos_prec == 4)
@@ -1822,9 +1902,14 @@ int paint(const PaintTiling *t, PaintScratch *s, int grid_prec, const void *x, c
             const int split = ngrids == 2;
             unsigned nb = slots < ntiles * ngrids ? slots : ntiles * ngrids;
             if (split) nb &= ~1u;
-            FG_CUDA(cudaFuncSetAttribute(paint_rot_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRotSmem));
-            paint_rot_kernel<<<nb, kPaintThreads, kRotSmem, st>>>(pp, s->hist, (const uint4 *)s->sorted, po, ntiles,
-                                                                  split);
+            FG_CUDA(cudaFuncSetAttribute(paint_rot_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRotSmem));
+            FG_CUDA(cudaFuncSetAttribute(paint_rot_kernel<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRotSmem));
+            if (ntiles * ngrids <= (unsigned)num_sms())
+                paint_rot_kernel<1024><<<nb, 1024, kRotSmem, st>>>(pp, s->hist, (const uint4 *)s->sorted, po, ntiles,
+                                                                   split);
+            else
+                paint_rot_kernel<512><<<nb, 512, kRotSmem, st>>>(pp, s->hist, (const uint4 *)s->sorted, po, ntiles,
+                                                                 split);
         } else {
             constexpr int T = kPaintThreads;
             const size_t smem = kAccBytes + sizeof(StageBuf) * (T / 32);

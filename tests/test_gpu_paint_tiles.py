@@ -120,3 +120,22 @@ def test_paint_fp64(fg, oracle_lib, Ng, kind, offset):
     g.p2k(cat)
     o.p2k(x, y, z, V)
     _close(g.exportf(), np.array(o.f), 1e-12)
+
+
+@pytest.mark.parametrize("Ng", [64, 96])
+@pytest.mark.parametrize("edge", [0.0, 0.5])
+def test_clump_at_a_tile_edge(fg, oracle_lib, Ng, edge):
+    """A clump whose base cells are the first of a tile (the box edge, or the
+    middle of the box where two tiles of Ng = 64 meet) reaches into the tile
+    below, whose fixed-point scale has to count it: with 200000 particles near
+    one cell an uncounted clump overflows that tile's 32-bit sums."""
+    L = 100.0
+    V = L ** 3
+    rng = np.random.default_rng(3)
+    p = L * edge + 0.2 * L / Ng * rng.random((3, 200_000)) + 0.1 * L / Ng
+    x, y, z = (np.asarray(a, dtype=np.float32).astype(np.float64) for a in p)
+    g = fg.Grid(Ng, L, precision="f32", host_view="lazy")
+    g.p2g(fg.Catalog(x, y, z, V), (0.0, 0.0, 0.0))
+    o = oracle_lib.Oracle(Ng, L)
+    o.p2g(x, y, z, V, (0.0, 0.0, 0.0))
+    _close(g.exportf(), np.array(o.f), 2e-5)
