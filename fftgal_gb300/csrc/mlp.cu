@@ -30,40 +30,118 @@ constexpr int kOffW1 = 0, kOffB1 = kOffW1 + kIn * kHid, kOffW2 = kOffB1 + kHid, 
               kOffB4 = kOffW4 + kHid * kOut, kNParams = kOffB4 + kOut;
 constexpr int kMlpThreads = 256, kMlpS = 32;  // samples per CTA round
 
-// a[s][j] = act(b[j] + sum_i x[s][i] W[i][j]) for S samples, cooperatively
-template <bool TANH>
-__device__ __forceinline__ void mlp_layer(const float *x, int nin, const float *W, const float *b, float *a, int nout,
-                                          int S) {
-    for (int e = threadIdx.x; e < S * nout; e += blockDim.x) {
-        const int s = e / nout, j = e - s * nout;
-        float z = b[j];
-        for (int i = 0; i < nin; ++i) z = fmaf(x[s * nin + i], W[i * nout + j], z);
-        a[e] = TANH ? tanhf(z) : z;
+// Gradient kernel.  Activations and deltas are kept as [unit][sample] with a pitch of
+// kPitch floats, W2 and W3 as [in][out] with a pitch of kWPitch (odd: a warp reads
+// a row or a column of either without bank conflicts).  Warp w takes samples 4w ..
+// 4w + 3, lane l the units l and l + 32 of a layer: 8 sums per thread and step from
+// one broadcast of 4 samples and two weights.  Every sum runs over its inputs (a
+// weight's gradient over the samples) in ascending order.  A training step at n =
+// 4096 (128 CTAs): 104 us with one output per thread at a time (two shared loads
+// per multiply-add, one scalar atomic per gradient and CTA; 68 us the kernel), 57 us
+// so.
+constexpr int kPitch = 36, kWPitch = 65;
+
+// out[l], out[l + 32] of the warp's 4 samples: z = b + sum_i x[i] W[i][.], i < nin
+template <int NIN>
+__device__ __forceinline__ void mlp_dense(const float *x, const float *W, int wp, const float *b, float (&z)[2][4],
+                                          int lane, int warp) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        z[0][q] = b[lane];
+        z[1][q] = b[lane + 32];
+    }
+#pragma unroll 8
+    for (int i = 0; i < NIN; ++i) {
+        const float4 v = *reinterpret_cast<const float4 *>(x + i * kPitch + 4 * warp);
+        const float w0 = W[i * wp + lane], w1 = W[i * wp + lane + 32];
+        z[0][0] = fmaf(v.x, w0, z[0][0]);
+        z[0][1] = fmaf(v.y, w0, z[0][1]);
+        z[0][2] = fmaf(v.z, w0, z[0][2]);
+        z[0][3] = fmaf(v.w, w0, z[0][3]);
+        z[1][0] = fmaf(v.x, w1, z[1][0]);
+        z[1][1] = fmaf(v.y, w1, z[1][1]);
+        z[1][2] = fmaf(v.z, w1, z[1][2]);
+        z[1][3] = fmaf(v.w, w1, z[1][3]);
     }
 }
 
-// delta of a hidden layer: d[s][i] = (sum_j dn[s][j] Wn[i][j]) (1 - a[s][i]^2)
-__device__ __forceinline__ void mlp_back(const float *dn, int nn, const float *Wn, const float *a, float *d, int S) {
-    for (int e = threadIdx.x; e < S * kHid; e += blockDim.x) {
-        const int s = e / kHid, i = e - s * kHid;
-        float g = 0.f;
-        for (int j = 0; j < nn; ++j) g = fmaf(dn[s * nn + j], Wn[i * nn + j], g);
-        d[e] = g * (1.f - a[e] * a[e]);
+__device__ __forceinline__ void mlp_put(float *a, const float (&z)[2][4], int lane, int warp) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+        *reinterpret_cast<float4 *>(a + (lane + 32 * h) * kPitch + 4 * warp) =
+            make_float4(z[h][0], z[h][1], z[h][2], z[h][3]);
+}
+
+// d[i] = (sum_j dn[j] W[i][j]) (1 - a[i]^2) for hidden units i = l, l + 32
+template <int NN>
+__device__ __forceinline__ void mlp_back(const float *dn, const float *W, int wp, const float *a, float *d, int lane,
+                                         int warp) {
+    float g[2][4] = {};
+#pragma unroll 8
+    for (int j = 0; j < NN; ++j) {
+        const float4 v = *reinterpret_cast<const float4 *>(dn + j * kPitch + 4 * warp);
+        const float w0 = W[lane * wp + j], w1 = W[(lane + 32) * wp + j];
+        g[0][0] = fmaf(v.x, w0, g[0][0]);
+        g[0][1] = fmaf(v.y, w0, g[0][1]);
+        g[0][2] = fmaf(v.z, w0, g[0][2]);
+        g[0][3] = fmaf(v.w, w0, g[0][3]);
+        g[1][0] = fmaf(v.x, w1, g[1][0]);
+        g[1][1] = fmaf(v.y, w1, g[1][1]);
+        g[1][2] = fmaf(v.z, w1, g[1][2]);
+        g[1][3] = fmaf(v.w, w1, g[1][3]);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const float4 v = *reinterpret_cast<const float4 *>(a + (lane + 32 * h) * kPitch + 4 * warp);
+        g[h][0] *= 1.f - v.x * v.x;
+        g[h][1] *= 1.f - v.y * v.y;
+        g[h][2] *= 1.f - v.z * v.z;
+        g[h][3] *= 1.f - v.w * v.w;
+    }
+    mlp_put(d, g, lane, warp);
+}
+
+// four neighbouring gradients; one vector atomic where the caller's array is 16-byte aligned
+__device__ __forceinline__ void grad_add4(float *g, float a, float b, float c, float d, bool vec) {
+    if (vec) {
+        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(g), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+    } else {
+        atomicAdd(g, a);
+        atomicAdd(g + 1, b);
+        atomicAdd(g + 2, c);
+        atomicAdd(g + 3, d);
     }
 }
 
-// gW[i][j] += sum_s x[s][i] d[s][j], gb[j] += sum_s d[s][j]
-__device__ __forceinline__ void mlp_accum(const float *x, int nin, const float *d, int nout, float *gW, float *gb,
-                                          int S) {
-    for (int e = threadIdx.x; e < nin * nout; e += blockDim.x) {
-        const int i = e / nout, j = e - i * nout;
-        float g = 0.f;
-        for (int s = 0; s < S; ++s) g = fmaf(x[s * nin + i], d[s * nout + j], g);
-        atomicAdd(&gW[e], g);
+// gW[i][j] += sum_s x[i][s] d[j][s] (64 outputs), gb[j] += sum_s d[j][s]: 4 x 4 weights per thread
+template <int NIN>
+__device__ __forceinline__ void mlp_accum64(const float *x, const float *d, float *gW, float *gb, bool vec) {
+    for (int t = threadIdx.x; t < (NIN + 3) / 4 * 16; t += kMlpThreads) {
+        const int j0 = 4 * (t & 15), i0 = 4 * (t >> 4);
+        float g[4][4] = {};
+#pragma unroll 2
+        for (int q = 0; q < kMlpS; q += 4) {
+            float4 u[4], v[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                u[e] = i0 + e < NIN ? *reinterpret_cast<const float4 *>(x + (i0 + e) * kPitch + q)
+                                    : make_float4(0.f, 0.f, 0.f, 0.f);
+                v[e] = *reinterpret_cast<const float4 *>(d + (j0 + e) * kPitch + q);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    g[i][j] = fmaf(u[i].w, v[j].w,
+                                   fmaf(u[i].z, v[j].z, fmaf(u[i].y, v[j].y, fmaf(u[i].x, v[j].x, g[i][j]))));
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (i0 + i < NIN) grad_add4(gW + (i0 + i) * kHid + j0, g[i][0], g[i][1], g[i][2], g[i][3], vec);
     }
-    for (int j = threadIdx.x; j < nout; j += blockDim.x) {
+    for (int j = threadIdx.x; j < kHid; j += kMlpThreads) {
         float g = 0.f;
-        for (int s = 0; s < S; ++s) g += d[s * nout + j];
+        for (int q = 0; q < kMlpS; ++q) g += d[j * kPitch + q];
         atomicAdd(&gb[j], g);
     }
 }
@@ -71,52 +149,89 @@ __device__ __forceinline__ void mlp_accum(const float *x, int nin, const float *
 // grad += d/dparams of sum_s scale * |y_s - t_s|^2 (scale = 1/n for the mean), loss += that sum
 __global__ void __launch_bounds__(kMlpThreads)
 mlp_grad_kernel(const float *__restrict__ params, const float *__restrict__ X, const float *__restrict__ T, long n,
-                float scale, float *__restrict__ grad, float *__restrict__ loss) {
+                float scale, float *__restrict__ grad, float *__restrict__ loss, int vec) {
     extern __shared__ __align__(16) float sm[];
-    float *P = sm;                       // kNParams
-    float *x0 = P + kNParams;            // [S][kIn]
-    float *a1 = x0 + kMlpS * kIn;        // [S][kHid]
-    float *a2 = a1 + kMlpS * kHid;
-    float *a3 = a2 + kMlpS * kHid;
-    float *y = a3 + kMlpS * kHid;        // [S][kOut] -> output deltas
-    float *d3 = y + kMlpS * kOut;        // [S][kHid]
-    float *d2 = d3 + kMlpS * kHid;
-    float *d1 = d2 + kMlpS * kHid;
-    __shared__ float lsum;
-    for (int e = threadIdx.x; e < kNParams; e += blockDim.x) P[e] = params[e];
-    if (threadIdx.x == 0) lsum = 0.f;
-    __syncthreads();
+    float *W2 = sm, *W3 = W2 + kHid * kWPitch;     // [64][kWPitch]
+    float *W1 = W3 + kHid * kWPitch;               // [5][64]
+    float *W4 = W1 + kIn * kHid;                   // [64][3]
+    float *b1 = W4 + kHid * kOut, *b2 = b1 + kHid, *b3 = b2 + kHid, *b4 = b3 + kHid;
+    float *x0 = b4 + 4;                            // [5][kPitch] (rows are 16-byte aligned)
+    float *a1 = x0 + kIn * kPitch;                 // [64][kPitch]
+    float *a2 = a1 + kHid * kPitch, *a3 = a2 + kHid * kPitch;
+    float *dy = a3 + kHid * kPitch;                // [3][kPitch] output deltas
+    float *d3 = dy + kOut * kPitch, *d2 = d3 + kHid * kPitch, *d1 = d2 + kHid * kPitch;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int e = tid; e < kHid * kHid; e += kMlpThreads) {
+        W2[e / kHid * kWPitch + e % kHid] = params[kOffW2 + e];
+        W3[e / kHid * kWPitch + e % kHid] = params[kOffW3 + e];
+    }
+    for (int e = tid; e < kIn * kHid; e += kMlpThreads) W1[e] = params[kOffW1 + e];
+    for (int e = tid; e < kHid * kOut; e += kMlpThreads) W4[e] = params[kOffW4 + e];
+    if (tid < kHid) {
+        b1[tid] = params[kOffB1 + tid];
+        b2[tid] = params[kOffB2 + tid];
+        b3[tid] = params[kOffB3 + tid];
+        if (tid < kOut) b4[tid] = params[kOffB4 + tid];
+    }
     for (long s0 = (long)blockIdx.x * kMlpS; s0 < n; s0 += (long)gridDim.x * kMlpS) {
         const int S = n - s0 < kMlpS ? (int)(n - s0) : kMlpS;
-        for (int e = threadIdx.x; e < S * kIn; e += blockDim.x) x0[e] = X[s0 * kIn + e];
-        __syncthreads();
-        mlp_layer<true>(x0, kIn, P + kOffW1, P + kOffB1, a1, kHid, S);
-        __syncthreads();
-        mlp_layer<true>(a1, kHid, P + kOffW2, P + kOffB2, a2, kHid, S);
-        __syncthreads();
-        mlp_layer<true>(a2, kHid, P + kOffW3, P + kOffB3, a3, kHid, S);
-        __syncthreads();
-        mlp_layer<false>(a3, kHid, P + kOffW4, P + kOffB4, y, kOut, S);
-        __syncthreads();
-        for (int e = threadIdx.x; e < S * kOut; e += blockDim.x) {
-            const float r = y[e] - T[s0 * kOut + e];
-            atomicAdd(&lsum, scale * r * r);
-            y[e] = 2.f * scale * r;  // output delta
+        __syncthreads();  // the parameters, or the previous round's reads
+        for (int e = tid; e < kMlpS * kIn; e += kMlpThreads) {
+            const int q = e / kIn, i = e - q * kIn;
+            x0[i * kPitch + q] = q < S ? X[s0 * kIn + e] : 0.f;
         }
         __syncthreads();
-        mlp_back(y, kOut, P + kOffW4, a3, d3, S);
+        float z[2][4];
+        // a warp's layers use its own 4 samples only: no barrier between them
+        mlp_dense<kIn>(x0, W1, kHid, b1, z, lane, warp);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) z[e >> 2][e & 3] = tanhf(z[e >> 2][e & 3]);
+        mlp_put(a1, z, lane, warp);
+        __syncwarp();
+        mlp_dense<kHid>(a1, W2, kWPitch, b2, z, lane, warp);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) z[e >> 2][e & 3] = tanhf(z[e >> 2][e & 3]);
+        mlp_put(a2, z, lane, warp);
+        __syncwarp();
+        mlp_dense<kHid>(a2, W3, kWPitch, b3, z, lane, warp);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) z[e >> 2][e & 3] = tanhf(z[e >> 2][e & 3]);
+        mlp_put(a3, z, lane, warp);
+        __syncwarp();
+        // outputs and their deltas: lane = (sample, output) of the warp's 12
+        float part = 0.f;
+        if (lane < 4 * kOut) {
+            const int q = 4 * warp + lane / kOut, o = lane % kOut;
+            float y = b4[o];
+#pragma unroll 8
+            for (int i = 0; i < kHid; ++i) y = fmaf(a3[i * kPitch + q], W4[i * kOut + o], y);
+            float r = 0.f;
+            if (q < S) r = y - T[(s0 + q) * kOut + o];
+            part = scale * r * r;
+            dy[o * kPitch + q] = 2.f * scale * r;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+        if (lane == 0) atomicAdd(loss, part);
+        __syncwarp();
+        mlp_back<kOut>(dy, W4, kOut, a3, d3, lane, warp);
+        __syncwarp();
+        mlp_back<kHid>(d3, W3, kWPitch, a2, d2, lane, warp);
+        __syncwarp();
+        mlp_back<kHid>(d2, W2, kWPitch, a1, d1, lane, warp);
         __syncthreads();
-        mlp_back(d3, kHid, P + kOffW3, a2, d2, S);
-        __syncthreads();
-        mlp_back(d2, kHid, P + kOffW2, a1, d1, S);
-        __syncthreads();
-        mlp_accum(a3, kHid, y, kOut, grad + kOffW4, grad + kOffB4, S);
-        mlp_accum(a2, kHid, d3, kHid, grad + kOffW3, grad + kOffB3, S);
-        mlp_accum(a1, kHid, d2, kHid, grad + kOffW2, grad + kOffB2, S);
-        mlp_accum(x0, kIn, d1, kHid, grad + kOffW1, grad + kOffB1, S);
-        __syncthreads();
+        mlp_accum64<kHid>(a2, d3, grad + kOffW3, grad + kOffB3, vec);
+        mlp_accum64<kHid>(a1, d2, grad + kOffW2, grad + kOffB2, vec);
+        mlp_accum64<kIn>(x0, d1, grad + kOffW1, grad + kOffB1, vec);
+        for (int e = tid; e < kHid * kOut + kOut; e += kMlpThreads) {
+            // W4 and b4: one of the 195 sums per thread
+            const int o = e % kOut, i = e / kOut;
+            float g = 0.f;
+            for (int q = 0; q < kMlpS; ++q)
+                g = i < kHid ? fmaf(a3[i * kPitch + q], dy[o * kPitch + q], g) : g + dy[o * kPitch + q];
+            atomicAdd(i < kHid ? &grad[kOffW4 + e] : &grad[kOffB4 + o], g);
+        }
     }
-    if (threadIdx.x == 0) atomicAdd(loss, lsum);
 }
 
 __global__ void mlp_adam_kernel(float *__restrict__ params, const float *__restrict__ grad, float *__restrict__ m,
@@ -132,39 +247,49 @@ __global__ void mlp_adam_kernel(float *__restrict__ params, const float *__restr
     params[e] -= lr * (mm / c1) / (sqrtf(vv / c2) + eps);
 }
 
-// one thread per sample: y = f(x)
-__global__ void __launch_bounds__(128)
+// y = f(x): a warp per sample, lane l the hidden units l and l + 32, the sums over
+// the inputs in ascending order.  The learned call at Ng = 256 (222 bins, 56 CTAs):
+// 536 -> 467 us against one thread per sample (two CTAs, the activations in local
+// memory: 67 us the kernel).
+constexpr int kFwdWarps = 4;
+__global__ void __launch_bounds__(32 * kFwdWarps)
 mlp_forward_kernel(const float *__restrict__ params, const float *__restrict__ X, long n, float *__restrict__ Y) {
-    __shared__ float P[kNParams];
+    __shared__ __align__(16) float P[kNParams];
+    __shared__ float act[kFwdWarps][2][kHid];
     for (int e = threadIdx.x; e < kNParams; e += blockDim.x) P[e] = params[e];
     __syncthreads();
-    const long s = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (s >= n) return;
-    float a[kHid], b[kHid];
-    for (int j = 0; j < kHid; ++j) {
-        float z = P[kOffB1 + j];
-        for (int i = 0; i < kIn; ++i) z = fmaf(X[s * kIn + i], P[kOffW1 + i * kHid + j], z);
-        a[j] = tanhf(z);
-    }
-    for (int j = 0; j < kHid; ++j) {
-        float z = P[kOffB2 + j];
-        for (int i = 0; i < kHid; ++i) z = fmaf(a[i], P[kOffW2 + i * kHid + j], z);
-        b[j] = tanhf(z);
-    }
-    for (int j = 0; j < kHid; ++j) {
-        float z = P[kOffB3 + j];
-        for (int i = 0; i < kHid; ++i) z = fmaf(b[i], P[kOffW3 + i * kHid + j], z);
-        a[j] = tanhf(z);
-    }
-    for (int o = 0; o < kOut; ++o) {
-        float z = P[kOffB4 + o];
-        for (int i = 0; i < kHid; ++i) z = fmaf(a[i], P[kOffW4 + i * kOut + o], z);
-        Y[s * kOut + o] = z;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float *a = act[warp][0], *b = act[warp][1];
+    for (long s = blockIdx.x * (long)kFwdWarps + warp; s < n; s += (long)gridDim.x * kFwdWarps) {
+        auto dense = [&](const float *x, int nin, int oW, int ob, float *out) {
+            float z0 = P[ob + lane], z1 = P[ob + lane + 32];
+#pragma unroll 8
+            for (int i = 0; i < nin; ++i) {
+                z0 = fmaf(x[i], P[oW + i * kHid + lane], z0);
+                z1 = fmaf(x[i], P[oW + i * kHid + lane + 32], z1);
+            }
+            out[lane] = tanhf(z0);
+            out[lane + 32] = tanhf(z1);
+            __syncwarp();
+        };
+        if (lane < kIn) b[lane] = X[s * kIn + lane];
+        __syncwarp();
+        dense(b, kIn, kOffW1, kOffB1, a);
+        dense(a, kHid, kOffW2, kOffB2, b);
+        dense(b, kHid, kOffW3, kOffB3, a);
+        if (lane < kOut) {
+            float z = P[kOffB4 + lane];
+#pragma unroll 8
+            for (int i = 0; i < kHid; ++i) z = fmaf(a[i], P[kOffW4 + i * kOut + lane], z);
+            Y[s * kOut + lane] = z;
+        }
+        __syncwarp();
     }
 }
 
 static size_t grad_smem() {
-    return sizeof(float) * ((size_t)kNParams + kMlpS * kIn + 3 * kMlpS * kHid + kMlpS * kOut + 3 * kMlpS * kHid);
+    return sizeof(float) * ((size_t)2 * kHid * kWPitch + kIn * kHid + kHid * kOut + 3 * kHid + 4 +
+                            (kIn + kOut + 6 * kHid) * kPitch);
 }
 
 }  // namespace fg
@@ -181,7 +306,8 @@ extern "C" int fftgal_mlp_grad(const float *params, const float *X, const float 
     FG_CUDA(cudaFuncSetAttribute(mlp_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     long nb = ceil_div(n, kMlpS);
     if (nb > 2L * num_sms()) nb = 2L * num_sms();
-    mlp_grad_kernel<<<(unsigned)nb, kMlpThreads, smem, st>>>(params, X, T, n, 1.0f / (float)n, grad, loss);
+    mlp_grad_kernel<<<(unsigned)nb, kMlpThreads, smem, st>>>(params, X, T, n, 1.0f / (float)n, grad, loss,
+                                                             reinterpret_cast<uintptr_t>(grad) % 16 == 0);
     FG_LAUNCHED(1);
     return OK;
 }
@@ -199,7 +325,9 @@ extern "C" int fftgal_mlp_adam(float *params, const float *grad, float *m, float
 
 extern "C" int fftgal_mlp_forward(const float *params, const float *X, long n, float *Y, void *stream) {
     if (!params || !X || !Y || n < 1) return set_error(ERR_ARG, "fftgal_mlp_forward: bad arguments");
-    mlp_forward_kernel<<<(unsigned)ceil_div(n, 128), 128, 0, static_cast<cudaStream_t>(stream)>>>(params, X, n, Y);
+    long nb = ceil_div(n, kFwdWarps);
+    if (nb > 4L * num_sms()) nb = 4L * num_sms();
+    mlp_forward_kernel<<<(unsigned)nb, 32 * kFwdWarps, 0, static_cast<cudaStream_t>(stream)>>>(params, X, n, Y);
     FG_LAUNCHED(1);
     return OK;
 }
