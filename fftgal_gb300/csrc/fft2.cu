@@ -11,7 +11,11 @@
 //           in-register FFT of length N2 and stores X[k1 + N1 k2].
 // One shared-memory round trip per pass (the Stockham kernels of fft.cu take
 // one per radix pass); the row pitches are padded so both shared-memory
-// phases are free of bank conflicts.  Length 2048 on the strided axes is
+// phases are free of bank conflicts.  The strided passes reach 4.6 (Ng = 1024) to
+// 5.9 TB/s (Ng = 512) of the 6.8 a copy does; DRAM moves each value once each way, and
+// what is left is the load and store phases of the 16 warps an SM holds, whose 64
+// registers of values leave no room for more.  Length 1024 on the strided axes takes
+// CTA pairs (fft2_cols1024_kernel), length 2048 is
 // 32 x 64 with the 64-point second step split over lane pairs
 // (fft2_cols2048_kernel).  Used for the forward r2c k pass and the strided
 // j/i passes of FP32 grids; other lengths use fft3.cu's mixed-radix passes or,
@@ -37,8 +41,40 @@ __host__ __device__ constexpr int bitrev(int x, int bits) {
     return r;
 }
 
+// u + t and u - t of a complex value in one packed operation each: they round as two
+// scalar operations do and take half the issue slots, but their results come later.
+// So the passes of large grids, which are short of issue slots, take them (Ng = 512 and
+// 1024, k pass: 362 and 3461 us against 369 and 3566; Ng = 256, j and i: 22 and 19
+// us against 24 and 22), and the short passes of small grids do not (Ng = 128: 5.8,
+// 5.9, 5.6 us against 6.2, 6.8, 6.8; Ng = 256, k: 24 against 28).
+__device__ __forceinline__ float2 add2(float2 u, float2 t) {
+    float2 r;
+    asm("{\n .reg .b64 a, b;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n add.rn.f32x2 a, a, b;\n"
+        " mov.b64 {%0, %1}, a;\n}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(u.x), "f"(u.y), "f"(t.x), "f"(t.y));
+    return r;
+}
+__device__ __forceinline__ float2 sub2(float2 u, float2 t) {
+    float2 r;
+    asm("{\n .reg .b64 a, b;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n sub.rn.f32x2 a, a, b;\n"
+        " mov.b64 {%0, %1}, a;\n}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(u.x), "f"(u.y), "f"(t.x), "f"(t.y));
+    return r;
+}
+
+// a b with the contraction written out: which product the compiler fuses depends on
+// the code around it, and the passes of every launch shape are to round alike
+template <bool FUSE_YX = false>
+__device__ __forceinline__ float2 cmul_fma(float2 a, float2 b) {
+    const float x = __fmaf_rn(a.x, b.x, -__fmul_rn(a.y, b.y));
+    const float y = FUSE_YX ? __fmaf_rn(a.y, b.x, __fmul_rn(a.x, b.y)) : __fmaf_rn(a.x, b.y, __fmul_rn(a.y, b.x));
+    return make_float2(x, y);
+}
+
 // in-register radix-2 FFT of length M <= 32, natural order in and out
-template <int M>
+template <int M, bool PACKED>
 __device__ __forceinline__ void reg_fft(float2 (&v)[M], int sign) {
     if constexpr (M > 1) {
         constexpr int B = ilog2c(M);
@@ -57,12 +93,15 @@ __device__ __forceinline__ void reg_fft(float2 (&v)[M], int sign) {
                 for (int s = 0; s < M; s += len) {
                     const float2 u = a[s + j];
                     float2 t = a[s + j + h];
-                    if (tix == 8)
+                    if (tix == 8) {  // t times sign i: the swap is free in scalar operations
                         t = cmul_si(t, sign);
-                    else if (tix != 0)
-                        t = cmul(t, w);
-                    a[s + j] = cadd(u, t);
-                    a[s + j + h] = csub(u, t);
+                        a[s + j] = cadd(u, t);
+                        a[s + j + h] = csub(u, t);
+                        continue;
+                    }
+                    if (tix != 0) t = cmul_fma(t, w);
+                    a[s + j] = PACKED ? add2(u, t) : cadd(u, t);
+                    a[s + j + h] = PACKED ? sub2(u, t) : csub(u, t);
                 }
             }
         }
@@ -70,6 +109,9 @@ __device__ __forceinline__ void reg_fft(float2 (&v)[M], int sign) {
         for (int i = 0; i < M; ++i) v[i] = a[i];
     }
 }
+
+template <int N> constexpr bool kColsPacked = N >= 256;  // N rows per column
+template <int M> constexpr bool kRowsPacked = M >= 256;  // M packed pairs per row
 
 __device__ __forceinline__ float2 twid(const float2 *__restrict__ W, int t, int sign) {
     float2 w = __ldg(&W[t]);
@@ -87,29 +129,41 @@ __device__ __forceinline__ void scale_all(float2 (&v)[M], float scale) {
 
 // ---- strided axis: C columns per CTA, threads = C * N2 ---------------------------
 // element n of column c of batch b: base + b*bs + n*es + c0 + c (complex units)
-// One tile: columns c0 .. c0 + C - 1 at `base` (= g + b*bs + c0), `left`
-// columns of them valid; threads t < nthr of the CTA (nthr >= C*N2).
-template <int N1, int N2>
-__device__ __forceinline__ void cols_tile(float2 *base, int left, long es, int logC, const float2 *__restrict__ W,
-                                          int sign, float scale, float2 *S, int t, int nthr) {
+// A load that stays where it is written: the compiler otherwise starts to transform the
+// first of 32 values before it has asked for the last ones (i pass at Ng = 1024: 3591 us
+// against 3621; up to length 512 plain loads are better, 420 us against 428).
+__device__ __forceinline__ float2 load2(const float2 *p) {
+    float2 v;
+    asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p) : "memory");
+    return v;
+}
+
+// One tile: columns c0 .. c0 + C - 1 at `base` (= g + b*bs + c0), of which
+// first .. left - 1 (at least one) are there; threads t < nthr of the CTA
+// (nthr >= C*N2).  The loads of the columns that are not there repeat one that is.
+template <int N1, int N2, int SIGN>
+__device__ __forceinline__ void cols_tile(float2 *base, int first, int left, long es, int logC,
+                                          const float2 *__restrict__ W, float scale, float2 *S, int t, int nthr) {
     const int C = 1 << logC;
     const int P = N1 * C + 8;  // shared pitch per n2
     if (t < C * N2) {
         const int c = t & (C - 1), n2 = t >> logC;
-        const bool ok = c < left;
+        const bool ok = c >= first && c < left;
         float2 v[N1];
+        const float2 *src = base + n2 * es + (ok ? c : max(first, 0));
+        const long step = N2 * es;
 #pragma unroll
-        for (int n1 = 0; n1 < N1; ++n1) {
-            const float2 *src = &base[(long)(N2 * n1 + n2) * es + c];
-            v[n1] = ok ? *src : make_float2(0.f, 0.f);
-        }
-        reg_fft<N1>(v, sign);
+        for (int n1 = 0; n1 < N1; ++n1, src += step) v[n1] = N1 * N2 > 512 ? load2(src) : *src;
+        reg_fft<N1, kColsPacked<N1 * N2>>(v, SIGN);
         if constexpr (N2 > 1) {
 #pragma unroll
-            for (int k1 = 1; k1 < N1; ++k1)
-                if (n2) v[k1] = cmul(v[k1], twid(W, n2 * k1, sign));
+            for (int k1 = 1; k1 < N1; ++k1) {
+                const float2 p = cmul_fma<true>(v[k1], twid(W, n2 * k1, SIGN));
+                v[k1] = n2 ? p : v[k1];
+            }
+            float2 *d = S + n2 * P + c;
 #pragma unroll
-            for (int k1 = 0; k1 < N1; ++k1) S[n2 * P + k1 * C + c] = v[k1];
+            for (int k1 = 0; k1 < N1; ++k1, d += C) *d = v[k1];
         } else {
             scale_all<N1>(v, scale);
             if (ok)
@@ -122,29 +176,121 @@ __device__ __forceinline__ void cols_tile(float2 *base, int left, long es, int l
         for (int s = t; s < C * N1; s += nthr) {
             const int c = s & (C - 1), k1 = s >> logC;
             float2 u[N2];
+            const float2 *q = S + k1 * C + c;
 #pragma unroll
-            for (int n2 = 0; n2 < N2; ++n2) u[n2] = S[n2 * P + k1 * C + c];
-            reg_fft<N2>(u, sign);
+            for (int n2 = 0; n2 < N2; ++n2, q += P) u[n2] = *q;
+            reg_fft<N2, kColsPacked<N1 * N2>>(u, SIGN);
             scale_all<N2>(u, scale);
-            if (c < left)
+            if (c >= first && c < left) {
+                float2 *d = base + k1 * es + c;
+                const long step = N1 * es;
 #pragma unroll
-                for (int k2 = 0; k2 < N2; ++k2) base[(long)(k1 + N1 * k2) * es + c] = u[k2];
+                for (int k2 = 0; k2 < N2; ++k2, d += step) *d = u[k2];
+            }
         }
     }
 }
 
-template <int N1, int N2>
+// tiles per batch: where all rows of a column share their alignment (es a multiple of
+// C: the i pass) a tile starts on a C-value boundary of memory, `off` columns early.  A
+// row of 16 columns is then one 128-byte line instead of five sectors of two lines
+// (i pass at Ng = 512: 583 us -> 364 with the loads below, j, which has no common
+// alignment, 571 -> 420; both grids), and the grids' Ng/2 + 1 = 1 mod 16 columns take
+// no more tiles than before.
+__host__ __device__ __forceinline__ int cols_tiles(int ncols, long es, int logC) {
+    const int C = 1 << logC;
+    return (ncols + C - 1 + ((es & (C - 1)) == 0 ? C - 1 : 0)) >> logC;
+}
+
+template <int N1, int N2, int SIGN>
 __global__ void __launch_bounds__(512)
 fft2_cols_kernel(float2 *g0, float2 *g1, int ncols, long es, long bs, int logC,
-                 const float2 *__restrict__ W, int sign, float scale) {
+                 const float2 *__restrict__ W, float scale) {
     extern __shared__ __align__(16) float2 S[];
-    const int C = 1 << logC;
-    const int ncb = (ncols + C - 1) >> logC;
+    const int ncb = cols_tiles(ncols, es, logC), C = 1 << logC;
     const int cb = blockIdx.x % ncb;
     const long batch = blockIdx.x / ncb;
-    float2 *g = blockIdx.y == 0 ? g0 : g1;
-    const int c0 = cb << logC;
-    cols_tile<N1, N2>(g + batch * bs + c0, ncols - c0, es, logC, W, sign, scale, S, threadIdx.x, blockDim.x);
+    float2 *g = (blockIdx.y == 0 ? g0 : g1) + batch * bs;
+    const int off = (es & (C - 1)) == 0 ? (int)((uintptr_t)g / sizeof(float2)) & (C - 1) : 0;
+    const int c0 = (cb << logC) - off;
+    if (c0 >= ncols) return;
+    cols_tile<N1, N2, SIGN>(g + c0, -c0, ncols - c0, es, logC, W, scale, S, threadIdx.x, blockDim.x);
+}
+
+// ---- strided axis of length 1024: a cluster of two CTAs per tile -------------------------
+// 16 columns of 1024 rows take 128 KB of shared memory, one CTA per SM, and nothing
+// runs while it loads or stores; 8 columns leave room for two CTAs but touch three
+// sectors per 64-byte row (rows start at odd multiples of 8 bytes).  Here two CTAs
+// share a tile of 16 columns: CTA q loads and transforms the rows 32 n1 + n2 of its 16
+// n2, sends Y[k1, n2] of the other's 16 k1 into that CTA's shared memory, and after
+// the cluster barrier transforms its own k1 over all n2.  66 KB per CTA, so two
+// tiles' halves share an SM.  The arithmetic is fft2_cols_kernel<32, 32>'s.  Both grids
+// at Ng = 1024: i pass 4.49 -> 3.59 ms, j pass 3.70 (8 columns) -> 3.76.  Prefetching
+// the next tile into L2 made it slower (4.2 ms), three CTAs of 80 registers 5.8.
+constexpr int kPairThreads = 256, kPairCols = 16, kPairPitch = 16 * kPairCols + 8;
+constexpr size_t kPairSmem = 32 * kPairPitch * sizeof(float2);
+
+template <int SIGN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 2)
+fft2_cols1024_kernel(float2 *g0, float2 *g1, int ncols, long es, long bs, const float2 *__restrict__ W, float scale) {
+    constexpr int C = kPairCols, P = kPairPitch;
+    extern __shared__ __align__(16) float2 S[];  // [n2][k1 of this CTA][c]
+    const int ncb = cols_tiles(ncols, es, 4);
+    const unsigned tile = blockIdx.x >> 1, rank = blockIdx.x & 1;
+    const int cb = tile % ncb;
+    const long batch = tile / ncb;
+    float2 *g = (blockIdx.y == 0 ? g0 : g1) + batch * bs;
+    const int off = (es & (C - 1)) == 0 ? (int)((uintptr_t)g / sizeof(float2)) & (C - 1) : 0;
+    const int c0 = cb * C - off;
+    if (c0 >= ncols) return;  // both CTAs of the tile
+    const int c = threadIdx.x & (C - 1), q = threadIdx.x >> 4, n2 = 16 * rank + q;
+    const bool ok = c0 + c >= 0 && c0 + c < ncols;
+    float2 *base = g + c0;
+    asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
+    {
+        float2 v[32];
+        const float2 *src = base + n2 * es + (ok ? c : max(-c0, 0));
+        const long step = 32 * es;
+#pragma unroll
+        for (int n1 = 0; n1 < 32; ++n1, src += step) v[n1] = load2(src);
+        reg_fft<32, true>(v, SIGN);
+#pragma unroll
+        for (int k1 = 1; k1 < 32; ++k1) {
+            const float2 p = cmul_fma<true>(v[k1], twid(W, n2 * k1, SIGN));
+            v[k1] = n2 ? p : v[k1];
+        }
+        asm volatile("barrier.cluster.wait;" ::: "memory");  // the other CTA is there
+        float2 *d = S + n2 * P + c;
+        uint32_t far;
+        asm("mapa.shared::cluster.u32 %0, %1, %2;"
+            : "=r"(far)
+            : "r"((uint32_t)__cvta_generic_to_shared(d)), "r"(rank ^ 1));
+        auto put = [&](const float2 *mine, const float2 *theirs) {
+#pragma unroll
+            for (int k = 0; k < 16; ++k) {
+                d[k * C] = mine[k];
+                asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(far + k * C * (int)sizeof(float2)),
+                             "f"(theirs[k].x), "f"(theirs[k].y)
+                             : "memory");
+            }
+        };
+        if (rank == 0)
+            put(v, v + 16);
+        else
+            put(v + 16, v);
+    }
+    asm volatile("barrier.cluster.arrive.release;\n barrier.cluster.wait.acquire;" ::: "memory");
+    float2 u[32];
+    const float2 *s = S + q * C + c;
+#pragma unroll
+    for (int m = 0; m < 32; ++m) u[m] = s[m * P];
+    reg_fft<32, true>(u, SIGN);
+    scale_all<32>(u, scale);
+    if (!ok) return;
+    float2 *d = base + (16 * rank + q) * es + c;
+    const long step = 32 * es;
+#pragma unroll
+    for (int k2 = 0; k2 < 32; ++k2, d += step) *d = u[k2];
 }
 
 // ---- strided axis of length 2048 = 32 x 64 ---------------------------------------------
@@ -177,7 +323,7 @@ fft2_cols2048_kernel(float2 *g0, float2 *g1, int ncols, long es, long bs, int lo
 #pragma unroll
         for (int n1 = 0; n1 < N1; ++n1)
             v[n1] = ok ? base[(long)(N2 * n1 + n2) * es + c] : make_float2(0.f, 0.f);
-        reg_fft<N1>(v, sign);
+        reg_fft<N1, true>(v, sign);
 #pragma unroll
         for (int k1 = 1; k1 < N1; ++k1)
             if (n2) v[k1] = cmul(v[k1], twid(W, n2 * k1, sign));
@@ -192,7 +338,7 @@ fft2_cols2048_kernel(float2 *g0, float2 *g1, int ncols, long es, long bs, int lo
     float2 u[32];
 #pragma unroll
     for (int m = 0; m < 32; ++m) u[m] = S[(2 * m + h) * P + k1 * C + c];
-    reg_fft<32>(u, sign);
+    reg_fft<32, true>(u, sign);
     const bool ok = c0 + c < ncols;
 #pragma unroll
     for (int k2 = 0; k2 < 32; ++k2) {
@@ -224,7 +370,7 @@ __device__ __forceinline__ void kr2c_tile(float *g, long nrows, int Ng_pad, int 
         float2 v[N1];
 #pragma unroll
         for (int n1 = 0; n1 < N1; ++n1) v[n1] = ok ? src[N2 * n1 + n2] : make_float2(0.f, 0.f);
-        reg_fft<N1>(v, -1);
+        reg_fft<N1, kRowsPacked<N1 * N2>>(v, -1);
 #pragma unroll
         for (int k1 = 1; k1 < N1; ++k1)
             if (n2) v[k1] = cmul(v[k1], twid(W, n2 * k1, -1));
@@ -243,7 +389,7 @@ __device__ __forceinline__ void kr2c_tile(float *g, long nrows, int Ng_pad, int 
         if (r < R) {
 #pragma unroll
             for (int n2 = 0; n2 < N2; ++n2) res[q][n2] = S[r * P + n2 * (N1 + 1) + k1];
-            reg_fft<N2>(res[q], -1);
+            reg_fft<N2, kRowsPacked<N1 * N2>>(res[q], -1);
         }
     }
     __syncthreads();
@@ -427,7 +573,7 @@ fft2_cols_tma_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_const
             float2 v[N1];
 #pragma unroll
             for (int n1 = 0; n1 < N1; ++n1) v[n1] = S[(N2 * n1 + n2) * C + c];
-            reg_fft<N1>(v, sign);
+            reg_fft<N1, true>(v, sign);
 #pragma unroll
             for (int k1 = 1; k1 < N1; ++k1)
                 if (n2) v[k1] = cmul(v[k1], twid(W, n2 * k1, sign));
@@ -455,7 +601,7 @@ fft2_cols_tma_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_const
                 issue(l + kTmaStages);
             }
         }
-        reg_fft<N2>(u, sign);
+        reg_fft<N2, true>(u, sign);
         float2 *base = (g ? g1 : g0) + (long)j * nh + kc0 + c;
 #pragma unroll
         for (int k2 = 0; k2 < N2; ++k2) base[(long)(k1 + N1 * k2) * es] = u[k2];
@@ -552,7 +698,7 @@ fft2_cols_tma_eo_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_co
             float2 v[N1];
 #pragma unroll
             for (int n1 = 0; n1 < N1; ++n1) v[n1] = S[(N2 * n1 + n2) * C + c];
-            reg_fft<N1>(v, sign);
+            reg_fft<N1, true>(v, sign);
 #pragma unroll
             for (int q = 1; q < N1; ++q)
                 if (n2) v[q] = cmul(v[q], twid(W, 2 * n2 * q, sign));
@@ -571,7 +717,7 @@ fft2_cols_tma_eo_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_co
                 issue(h + kTmaStages);
             }
         }
-        reg_fft<N2>(u, sign);  // u[k2] = transform of this parity at k1 + 32 k2
+        reg_fft<N2, true>(u, sign);  // u[k2] = transform of this parity at k1 + 32 k2
         if ((h & 1) == 0) {
 #pragma unroll
             for (int q = 0; q < N2; ++q) E[q] = u[q];
@@ -639,20 +785,19 @@ bool fft2_supported(int Ng, int prec) {
 
 #define FG_COLS_CASE(A, B)                                                                                 \
     if (N1 == A && N2 == B) {                                                                             \
-        FG_CUDA(cudaFuncSetAttribute(fft2_cols_kernel<A, B>, cudaFuncAttributeMaxDynamicSharedMemorySize,   \
-                                     (int)smem));                                                         \
-        fft2_cols_kernel<A, B><<<grid, threads, smem, s>>>((float2 *)g0, (float2 *)g1, ncols, es, bs,      \
-                                                           logC, (const float2 *)W, sign, (float)scale);   \
+        const auto kernel = sign < 0 ? fft2_cols_kernel<A, B, -1> : fft2_cols_kernel<A, B, 1>;             \
+        FG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));     \
+        kernel<<<grid, threads, smem, s>>>((float2 *)g0, (float2 *)g1, ncols, es, bs, logC,                \
+                                           (const float2 *)W, (float)scale);                               \
         FG_LAUNCHED(1);                                                                                    \
         return OK;                                                                                         \
     }
 
-// C columns per CTA: threads = C*N2 around 256, C >= 8 for 64-byte rows;
-// along a widely strided axis (the i pass) C = 16, so every row access is a
-// 128-byte run (measured 15 % faster at Ng = 1024; the j pass is faster with
-// C = 8 and two CTAs per SM)
+// C columns per CTA: threads = C*N2 around 256, C >= 8 for 64-byte rows; along a
+// widely strided axis (the i pass) and at length 1024 (CTA pairs) C = 16, so a row
+// access is a 128-byte run
 static int cols_default_logC(int N2, bool wide) {
-    int logC = wide ? 4 : 3;
+    int logC = wide || N2 == 32 ? 4 : 3;
     while ((1 << logC) * N2 < 256 && logC < 5) ++logC;
     while ((1 << logC) * N2 > 512 && logC > 0) --logC;
     return logC;
@@ -838,12 +983,20 @@ int fft2_cols(int N, const void *W, void *g0, void *g1, int ngrids, int ncols, l
     const int C = 1 << logC;
     const int threads = C * N2;
     const size_t smem = cols_smem(N1, N2, logC, paired);
-    const long ncb = ceil_div(ncols, C);
-    dim3 grid((unsigned)(ncb * nbatch), ngrids);
+    dim3 grid((unsigned)((paired ? ceil_div(ncols, C) : cols_tiles(ncols, es, logC)) * nbatch), ngrids);
     if (paired) {
         FG_CUDA(cudaFuncSetAttribute(fft2_cols2048_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         fft2_cols2048_kernel<<<grid, threads, smem, s>>>((float2 *)g0, (float2 *)g1, ncols, es, bs, logC,
                                                          (const float2 *)W, sign, (float)scale);
+        FG_LAUNCHED(1);
+        return OK;
+    }
+    if (N == 1024 && logC == 4) {
+        const auto kernel = sign < 0 ? fft2_cols1024_kernel<-1> : fft2_cols1024_kernel<1>;
+        FG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmem));
+        grid.x *= 2;
+        kernel<<<grid, kPairThreads, kPairSmem, s>>>((float2 *)g0, (float2 *)g1, ncols, es, bs, (const float2 *)W,
+                                                     (float)scale);
         FG_LAUNCHED(1);
         return OK;
     }
