@@ -191,28 +191,16 @@ __device__ __forceinline__ void cols_tile(float2 *base, int first, int left, lon
     }
 }
 
-// tiles per batch: where all rows of a column share their alignment (es a multiple of
-// C: the i pass) a tile starts on a C-value boundary of memory, `off` columns early.  A
-// row of 16 columns is then one 128-byte line instead of five sectors of two lines
-// (i pass at Ng = 512: 583 us -> 364 with the loads below, j, which has no common
-// alignment, 571 -> 420; both grids), and the grids' Ng/2 + 1 = 1 mod 16 columns take
-// no more tiles than before.
-__host__ __device__ __forceinline__ int cols_tiles(int ncols, long es, int logC) {
-    const int C = 1 << logC;
-    return (ncols + C - 1 + ((es & (C - 1)) == 0 ? C - 1 : 0)) >> logC;
-}
-
 template <int N1, int N2, int SIGN>
 __global__ void __launch_bounds__(512)
 fft2_cols_kernel(float2 *g0, float2 *g1, int ncols, long es, long bs, int logC,
                  const float2 *__restrict__ W, float scale) {
     extern __shared__ __align__(16) float2 S[];
-    const int ncb = cols_tiles(ncols, es, logC), C = 1 << logC;
+    const int ncb = cols_tiles(ncols, es, logC);
     const int cb = blockIdx.x % ncb;
     const long batch = blockIdx.x / ncb;
     float2 *g = (blockIdx.y == 0 ? g0 : g1) + batch * bs;
-    const int off = (es & (C - 1)) == 0 ? (int)((uintptr_t)g / sizeof(float2)) & (C - 1) : 0;
-    const int c0 = (cb << logC) - off;
+    const int c0 = (cb << logC) - cols_offset(g, es, logC);
     if (c0 >= ncols) return;
     cols_tile<N1, N2, SIGN>(g + c0, -c0, ncols - c0, es, logC, W, scale, S, threadIdx.x, blockDim.x);
 }
@@ -240,8 +228,7 @@ fft2_cols1024_kernel(float2 *g0, float2 *g1, int ncols, long es, long bs, const 
     const int cb = tile % ncb;
     const long batch = tile / ncb;
     float2 *g = (blockIdx.y == 0 ? g0 : g1) + batch * bs;
-    const int off = (es & (C - 1)) == 0 ? (int)((uintptr_t)g / sizeof(float2)) & (C - 1) : 0;
-    const int c0 = cb * C - off;
+    const int c0 = cb * C - cols_offset(g, es, 4);
     if (c0 >= ncols) return;  // both CTAs of the tile
     const int c = threadIdx.x & (C - 1), q = threadIdx.x >> 4, n2 = 16 * rank + q;
     const bool ok = c0 + c >= 0 && c0 + c < ncols;

@@ -14,13 +14,14 @@
 //   alike: A[k] = (Z[k] + conj Z[N-k]) / 2, B[k] = (Z[k] - conj Z[N-k]) / 2i.
 // The general kernels of fft.cu (radix passes through shared memory with
 // run-time strides) remain for other lengths and FP64 grids.
-// Measured (GB300, both interlacing grids): whole calls at Ng = 384 6.27 -> 1.69 ms
-// and at Ng = 225 2.95 -> 0.51 ms (k pass 1402 / 1083 us and j + i passes 3655 /
-// 1493 us in the general kernels: run-time divisions per element, one memory
-// round trip per radix and O(R^2) odd butterflies from constant memory).  128
-// registers for the longest lengths hold the kernels to two CTAs of 256 threads
-// per SM; 16 columns per CTA keep global rows at 128 bytes and shared accesses
-// free of conflicts without padding.
+// Measured (GB300, both interlacing grids, us): Ng = 384 k 1402 -> 266, j + i 3655 -> 404
+// and Ng = 225 1083 -> 57, 1493 -> 94 (in the general kernels: run-time divisions per
+// element, one memory round trip per radix and O(R^2) odd butterflies from constant
+// memory).  128 registers for the longest lengths hold the kernels to two CTAs of 256
+// threads per SM, whose load and store phases bound them (Ng = 384: 3.4 and 4.5 TB/s
+// of the 6.8 a copy does); 16 columns per CTA, on a 128-byte boundary where the rows
+// share one (cols_tiles), keep global rows at 128 bytes and shared accesses free of
+// conflicts without padding.
 #include "internal.h"
 #include "common.cuh"
 #include "regfft.cuh"
@@ -30,27 +31,25 @@
 namespace fg {
 
 constexpr int kF3Threads = 256;
-constexpr int kF3Cols = 16;  // columns per CTA (a power of two)
+constexpr int kF3LogCols = 4, kF3Cols = 1 << kF3LogCols;  // columns per CTA
 
 #define FG_F3_LENGTHS(X)                                                                                       \
     X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16) X(18) X(20) X(21) \
         X(22) X(24) X(25) X(26) X(27) X(28) X(30) X(32)
 
 // ---- strided axis ---------------------------------------------------------------------
+// columns first .. left - 1 of a tile are there (at least one); the others load it too
 // step 1: x[N2 n1 + n2] of column c -> S[n2 P + k1 C + c]
 template <int M>
-__device__ __noinline__ void cols_step1(const float2 *__restrict__ base, float2 *S, int left, long es, int N2, int P,
-                                        const float2 *__restrict__ W, float sgn) {
+__device__ __noinline__ void cols_step1(const float2 *__restrict__ base, float2 *S, int first, int left, long es,
+                                        int N2, int P, const float2 *__restrict__ W, float sgn) {
     for (int s = threadIdx.x; s < kF3Cols * N2; s += kF3Threads) {
         const int c = s & (kF3Cols - 1), n2 = s / kF3Cols;
-        const float2 *src = base + (long)n2 * es + c;
+        const float2 *src = base + (long)n2 * es + (c >= first && c < left ? c : max(first, 0));
         const long st = (long)N2 * es;
         float2 v[M];
 #pragma unroll
-        for (int n = 0; n < M; ++n) {
-            v[n] = c < left ? *src : make_float2(0.f, 0.f);
-            src += st;
-        }
+        for (int n = 0; n < M; ++n, src += st) v[n] = *src;
 #pragma unroll
         for (int n = 0; n < M; ++n) v[n].y *= sgn;
         fft_reg<M>(v);
@@ -62,8 +61,8 @@ __device__ __noinline__ void cols_step1(const float2 *__restrict__ base, float2 
 
 // step 2: S -> X[k1 + N1 k2] scale
 template <int M>
-__device__ __noinline__ void cols_step2(float2 *__restrict__ base, const float2 *S, int left, long es, int N1, int P,
-                                        float sgn, float scale) {
+__device__ __noinline__ void cols_step2(float2 *__restrict__ base, const float2 *S, int first, int left, long es,
+                                        int N1, int P, float sgn, float scale) {
     for (int s = threadIdx.x; s < kF3Cols * N1; s += kF3Threads) {
         const int c = s & (kF3Cols - 1), k1 = s / kF3Cols;
         const float2 *src = S + s;
@@ -71,7 +70,7 @@ __device__ __noinline__ void cols_step2(float2 *__restrict__ base, const float2 
 #pragma unroll
         for (int n = 0; n < M; ++n) u[n] = src[n * P];
         fft_reg<M>(u);
-        if (c >= left) continue;
+        if (c < first || c >= left) continue;
         float2 *dst = base + (long)k1 * es + c;
         const long st = (long)N1 * es;
         const float sy = scale * sgn;
@@ -87,21 +86,23 @@ __global__ void __launch_bounds__(kF3Threads, 2)
 fft3_cols_kernel(float2 *g0, float2 *g1, int ncols, long es, long bs, int N1, int N2, int P,
                  const float2 *__restrict__ W, float sgn, float scale) {
     extern __shared__ __align__(16) float2 f3_smem[];
-    const int ncb = (ncols + kF3Cols - 1) / kF3Cols;
+    const int ncb = cols_tiles(ncols, es, kF3LogCols);
     const int cb = blockIdx.x % ncb;
     const long batch = blockIdx.x / ncb;
-    const int c0 = cb * kF3Cols;
-    float2 *base = (blockIdx.y == 0 ? g0 : g1) + batch * bs + c0;
+    float2 *base = (blockIdx.y == 0 ? g0 : g1) + batch * bs;
+    const int c0 = cb * kF3Cols - cols_offset(base, es, kF3LogCols);
+    if (c0 >= ncols) return;
+    base += c0;
     switch (N1) {
 #define FG_CASE(M) \
-    case M: cols_step1<M>(base, f3_smem, ncols - c0, es, N2, P, W, sgn); break;
+    case M: cols_step1<M>(base, f3_smem, -c0, ncols - c0, es, N2, P, W, sgn); break;
         FG_F3_LENGTHS(FG_CASE)
 #undef FG_CASE
     }
     __syncthreads();
     switch (N2) {
 #define FG_CASE(M) \
-    case M: cols_step2<M>(base, f3_smem, ncols - c0, es, N1, P, sgn, scale); break;
+    case M: cols_step2<M>(base, f3_smem, -c0, ncols - c0, es, N1, P, sgn, scale); break;
         FG_F3_LENGTHS(FG_CASE)
 #undef FG_CASE
     }
@@ -111,6 +112,7 @@ fft3_cols_kernel(float2 *g0, float2 *g1, int ncols, long es, long bs, int N1, in
 // the layout of a CTA's R row pairs: S[(r N2 + n2) Q + k1], D[r PZ + n]
 struct Rows {
     int N, N1, N2, Q, PZ, R;
+    uint32_t inv_n, inv_nh;  // e / N and e / (N/2 + 1) as the high word of a product
 };
 
 // step 1 of the forward pass: rows 2r and 2r + 1 of g (from row0; nrows in all)
@@ -195,7 +197,7 @@ fft3_k_r2c_kernel(float *g0, float *g1, long nrows, int Ng_pad, Rows d, const fl
     __syncthreads();
     const int nh = d.N / 2 + 1;
     for (int e = threadIdx.x; e < d.R * nh; e += kF3Threads) {
-        const int r = e / nh, k = e - r * nh;
+        const int r = (int)__umulhi(e, d.inv_nh), k = e - r * nh;
         const long row = row0 + 2 * r;
         if (row >= nrows) break;
         const float2 z = D[r * d.PZ + k], y = D[r * d.PZ + (k ? d.N - k : 0)];
@@ -215,7 +217,7 @@ fft3_k_c2r_kernel(float *g0, float *g1, long nrows, int Ng_pad, Rows d, const fl
     // conj Z, Z = A + i B of a row pair over all N wavenumbers; the imaginary parts
     // of k = 0 and the Nyquist column are ignored
     for (int e = threadIdx.x; e < d.R * nh; e += kF3Threads) {
-        const int r = e / nh, k = e - r * nh;
+        const int r = (int)__umulhi(e, d.inv_nh), k = e - r * nh;
         const long row = row0 + 2 * r;
         const float2 *in = reinterpret_cast<const float2 *>(g + row * Ng_pad) + k;
         float2 a = row < nrows ? *in : make_float2(0.f, 0.f);
@@ -235,7 +237,7 @@ fft3_k_c2r_kernel(float *g0, float *g1, long nrows, int Ng_pad, Rows d, const fl
     rows_fft2(S, D, d);
     __syncthreads();
     for (int e = threadIdx.x; e < d.R * N; e += kF3Threads) {
-        const int r = e / N, n = e - r * N;
+        const int r = (int)__umulhi(e, d.inv_n), n = e - r * N;
         const long row = row0 + 2 * r;
         if (row >= nrows) break;
         const float2 z = D[r * d.PZ + n];
@@ -288,6 +290,9 @@ static Rows rows_shape(int N, int N1, int N2) {
     const size_t one = (size_t)(N2 * d.Q + d.PZ) * sizeof(float2);
     while (d.R > 1 && d.R * one > 64 * 1024) --d.R;
     if (d.R > 16) d.R = 16;
+    // ceil(2^32 / v): exact for e < 2^32 / v, and e < R v <= 2^14
+    d.inv_n = (uint32_t)((0x100000000ull + N - 1) / N);
+    d.inv_nh = (uint32_t)((0x100000000ull + N / 2) / (N / 2 + 1));
     return d;
 }
 
@@ -302,7 +307,7 @@ int fft3_cols(int N, const void *W, void *g0, void *g1, int ngrids, int ncols, l
     if (!split3(N, &N1, &N2)) return set_error(ERR_UNSUPPORTED, "fft3_cols: N=%d", N);
     const size_t smem = cols3_smem(N1, N2, &P);
     FG_CUDA(cudaFuncSetAttribute(fft3_cols_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    const dim3 grid((unsigned)(ceil_div(ncols, kF3Cols) * nbatch), ngrids);
+    const dim3 grid((unsigned)(cols_tiles(ncols, es, kF3LogCols) * nbatch), ngrids);
     fft3_cols_kernel<<<grid, kF3Threads, smem, s>>>((float2 *)g0, (float2 *)g1, ncols, es, bs, N1, N2, P,
                                                     (const float2 *)W, sign > 0 ? -1.f : 1.f, (float)scale);
     FG_LAUNCHED(1);
