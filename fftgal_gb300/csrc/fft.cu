@@ -518,14 +518,16 @@ static int scale_grids(const FftPlan *p, void *const *grids, int ngrids, double 
     return OK;
 }
 
-// The k pass: forward, powers of two take fft2.cu's packed rows (half-length
-// transforms); everything else, and every backward pass, the row pairs of
-// fft3.cu where the length splits; the general kernels below otherwise (c2r
-// at Ng = 512: 733 us there, at Ng = 384 both grids forward 1402 us).
+// The k pass: powers of two take fft2.cu's packed rows (half-length transforms);
+// other lengths the row pairs of fft3.cu where they split; the general kernels
+// below do the rest (c2r at Ng = 512: 733 us there, 518 in fft3.cu, 215 in fft2.cu;
+// both grids forward at Ng = 384: 1402 us there, 266 in fft3.cu).
 static int k_pass(const FftPlan *p, void *const *grids, int ngrids, bool forward, cudaStream_t s, double scale = 1) {
-    if (forward && fft2_supported(p->Ng, p->prec))
-        return fft2_k_r2c(p->Ng, p->half.tw, p->rtw, grids[0], ngrids > 1 ? grids[1] : grids[0], ngrids, s,
-                          p->tune[0]);
+    if (fft2_supported(p->Ng, p->prec)) {
+        void *g1 = ngrids > 1 ? grids[1] : grids[0];
+        return forward ? fft2_k_r2c(p->Ng, p->half.tw, p->rtw, grids[0], g1, ngrids, s, p->tune[0])
+                       : fft2_k_c2r(p->Ng, p->half.tw, p->rtw, grids[0], g1, ngrids, scale, s);
+    }
     if (fft3_supported(p->Ng, p->prec))
         return fft3_k(p->Ng, p->axis.tw, grids[0], ngrids > 1 ? grids[1] : grids[0], ngrids, forward, scale, s);
     const long nrows = (long)p->Ng * p->Ng;

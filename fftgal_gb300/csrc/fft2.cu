@@ -17,8 +17,8 @@
 // registers of values leave no room for more.  Length 1024 on the strided axes takes
 // CTA pairs (fft2_cols1024_kernel), length 2048 is
 // 32 x 64 with the 64-point second step split over lane pairs
-// (fft2_cols2048_kernel).  Used for the forward r2c k pass and the strided
-// j/i passes of FP32 grids; other lengths use fft3.cu's mixed-radix passes or,
+// (fft2_cols2048_kernel).  Used for the k pass both ways (r2c, c2r) and the
+// strided j/i passes of FP32 grids; other lengths use fft3.cu's mixed-radix passes or,
 // where those do not apply (FP64 grids among them), the general kernels of fft.cu.
 #include "internal.h"
 #include "common.cuh"
@@ -418,6 +418,60 @@ fft2_k_r2c_kernel(float *g0, float *g1, long nrows, int Ng_pad, int R,
     extern __shared__ __align__(16) float2 S[];
     kr2c_tile<N1, N2>(blockIdx.y == 0 ? g0 : g1, nrows, Ng_pad, R, (long)blockIdx.x * R, W, rtw, S, threadIdx.x,
                       blockDim.x);
+}
+
+// ---- k axis, backward c2r: R rows per CTA, threads = R * N2 --------------------------
+// The packed row z[m] = x[2m] + i x[2m+1] is the backward transform, of length M = Ng / 2,
+// of  Z[k] = X[k] + conj X[M-k] + i W_Ng^-k (X[k] - conj X[M-k]).  A thread reads X[k] and
+// X[M-k] for each of its k = N2 n1 + n2 (the second reading of a row hits L1), so Z
+// needs no trip through shared memory; step 2 stores to the rows.  The imaginary
+// parts of X[0] and X[M] are ignored, and the row padding keeps its values, scaled
+// like the rest of the grid.  One grid of Ng = 512: 518 us with the row pairs of
+// fft3.cu (whole-length transforms, four trips through shared memory), about 215 here.
+template <int N1, int N2>
+__global__ void __launch_bounds__(512)
+fft2_k_c2r_kernel(float *g0, float *g1, long nrows, int Ng_pad, int R, const float2 *__restrict__ W,
+                  const float2 *__restrict__ rtw, float scale) {
+    constexpr int M = N1 * N2, P = N2 * (N1 + 1);
+    extern __shared__ __align__(16) float2 S[];
+    float *g = blockIdx.y == 0 ? g0 : g1;
+    const long row0 = (long)blockIdx.x * R;
+    const int t = threadIdx.x, n2 = t % N2, rt = t / N2;
+    const bool ok = row0 + rt < nrows;
+    float2 *row = reinterpret_cast<float2 *>(g + (ok ? row0 + rt : row0) * Ng_pad);
+    const float2 end = row[M];
+    {
+        float2 v[N1];
+#pragma unroll
+        for (int n1 = 0; n1 < N1; ++n1) {
+            const int m = N2 * n1 + n2;
+            float2 a = row[m], b = cconj(row[M - m]);
+            if (m == 0) a.y = b.y = 0.f;
+            const float2 A = cadd(a, b), B = cmul(csub(a, b), cconj(__ldg(&rtw[m])));
+            v[n1] = make_float2(A.x - B.y, A.y + B.x);
+        }
+        reg_fft<N1, kRowsPacked<M>>(v, 1);
+        float2 *d = S + rt * P + n2 * (N1 + 1);
+#pragma unroll
+        for (int k1 = 0; k1 < N1; ++k1) {
+            const float2 p = k1 ? cmul_fma<true>(v[k1], twid(W, n2 * k1, 1)) : v[k1];
+            d[k1] = n2 ? p : v[k1];
+        }
+    }
+    __syncthreads();
+    for (int s = t; s < R * N1; s += blockDim.x) {
+        const int k1 = s % N1, r = s / N1;
+        if (row0 + r >= nrows) break;
+        float2 u[N2];
+#pragma unroll
+        for (int q = 0; q < N2; ++q) u[q] = S[r * P + q * (N1 + 1) + k1];
+        reg_fft<N2, kRowsPacked<M>>(u, 1);
+        scale_all<N2>(u, scale);
+        float2 *out = reinterpret_cast<float2 *>(g + (row0 + r) * Ng_pad) + k1;
+#pragma unroll
+        for (int k2 = 0; k2 < N2; ++k2) out[N1 * k2] = u[k2];
+    }
+    if (ok && n2 == 0) row[M] = make_float2(end.x * scale, end.y * scale);
 }
 
 // ---- widely strided axis (the i pass), columns staged by TMA ----------------------------------
@@ -1040,6 +1094,39 @@ int fft2_k_r2c(int Ng, const void *W, const void *rtw, void *g0, void *g1, int n
     FG_K_CASE(32, 16)
     FG_K_CASE(32, 32)
     return set_error(ERR_UNSUPPORTED, "fft2_k_r2c: no kernel for %d x %d", N1, N2);
+}
+#undef FG_K_CASE
+
+#define FG_K_CASE(A, B)                                                                                    \
+    if (N1 == A && N2 == B) {                                                                             \
+        FG_CUDA(cudaFuncSetAttribute(fft2_k_c2r_kernel<A, B>, cudaFuncAttributeMaxDynamicSharedMemorySize,  \
+                                     (int)smem));                                                         \
+        fft2_k_c2r_kernel<A, B><<<grid, R * N2, smem, s>>>((float *)g0, (float *)g1, nrows, Ng + 2, R,     \
+                                                           (const float2 *)W, (const float2 *)rtw,         \
+                                                           (float)scale);                                  \
+        FG_LAUNCHED(1);                                                                                    \
+        return OK;                                                                                         \
+    }
+
+int fft2_k_c2r(int Ng, const void *W, const void *rtw, void *g0, void *g1, int ngrids, double scale, cudaStream_t s) {
+    FG_TRY(ensure_w32());
+    int N1, N2;
+    if (!split2(Ng / 2, &N1, &N2)) return set_error(ERR_UNSUPPORTED, "fft2_k_c2r: Ng=%d", Ng);
+    const long nrows = (long)Ng * Ng;
+    const int R = k_default_rows(N2);
+    const size_t smem = (size_t)R * N2 * (N1 + 1) * sizeof(float2);
+    const dim3 grid((unsigned)ceil_div(nrows, R), ngrids);
+    FG_K_CASE(2, 1)
+    FG_K_CASE(2, 2)
+    FG_K_CASE(4, 2)
+    FG_K_CASE(4, 4)
+    FG_K_CASE(8, 4)
+    FG_K_CASE(8, 8)
+    FG_K_CASE(16, 8)
+    FG_K_CASE(16, 16)
+    FG_K_CASE(32, 16)
+    FG_K_CASE(32, 32)
+    return set_error(ERR_UNSUPPORTED, "fft2_k_c2r: no kernel for %d x %d", N1, N2);
 }
 #undef FG_K_CASE
 

@@ -1,7 +1,6 @@
 // Mixed-radix FFT passes of FP32 grids (sm_103a): lengths N = N1 N2 with N1, N2
 // <= 32 and prime factors up to 13, e.g. 96, 225, 384, 500 -- the sizes that the
-// power-of-two passes of fft2.cu do not take -- and the backward k pass (c2r) of
-// every such length, powers of two included.
+// power-of-two passes of fft2.cu do not take.
 //
 // As in fft2.cu a transform is two in-register FFTs around one trip through
 // shared memory,

@@ -92,6 +92,7 @@ int fft2_cols(int N, const void *W, void *g0, void *g1, int ngrids, int ncols, l
               long nbatch, int sign, cudaStream_t s, int logC_req = -1, double scale = 1);
 int fft2_k_r2c(int Ng, const void *W, const void *rtw, void *g0, void *g1, int ngrids, cudaStream_t s,
                int R_req = 0);
+int fft2_k_c2r(int Ng, const void *W, const void *rtw, void *g0, void *g1, int ngrids, double scale, cudaStream_t s);
 // launch shape `v` of pass `which` (0 = k rows per CTA, 1 = j / 2 = i log2
 // columns per CTA) is launchable for Ng; the built-in choice of each pass
 bool fft2_valid_shape(int Ng, int which, int v);
