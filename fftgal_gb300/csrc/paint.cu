@@ -372,20 +372,9 @@ __global__ void scan_block_sums(const uint32_t *__restrict__ a, long n, uint32_t
     if (threadIdx.x == 0) bsum[blockIdx.x] = tot;
 }
 
-__global__ void scan_top(uint32_t *bsum, long nb) {
-    __shared__ uint32_t ws[32];
-    __shared__ uint32_t tot;
-    uint32_t carry = 0;
-    for (long c0 = 0; c0 < nb; c0 += blockDim.x) {
-        const long i = c0 + threadIdx.x;
-        const uint32_t v = i < nb ? bsum[i] : 0;
-        const uint32_t e = block_exclusive_scan(v, ws, &tot);
-        if (i < nb) bsum[i] = carry + e;
-        carry += tot;
-        __syncthreads();
-    }
-}
-
+// a block adds up the sums of the blocks before it itself: a launch less than a scan
+// of the sums in between (Ng = 256, 27649 entries: 13 us against 17; one CTA for all of
+// them, as for short arrays, 24)
 __global__ void scan_apply(uint32_t *__restrict__ a, uint32_t *__restrict__ cursor, long n,
                            const uint32_t *__restrict__ bsum) {
     __shared__ uint32_t ws[32];
@@ -398,7 +387,11 @@ __global__ void scan_apply(uint32_t *__restrict__ a, uint32_t *__restrict__ curs
         v[i] = base + i < n ? a[base + i] : 0;
         s += v[i];
     }
-    uint32_t e = block_exclusive_scan(s, ws, &tot) + bsum[blockIdx.x];
+    uint32_t before = 0;
+    for (unsigned i = threadIdx.x; i < blockIdx.x; i += blockDim.x) before += bsum[i];
+    block_exclusive_scan(before, ws, &tot);
+    before = tot;
+    uint32_t e = before + block_exclusive_scan(s, ws, &tot);
 #pragma unroll
     for (int i = 0; i < kScanPer; ++i) {
         if (base + i < n) a[base + i] = cursor[base + i] = e;
@@ -440,9 +433,8 @@ static int exclusive_scan(uint32_t *a, uint32_t *cursor, long n, uint32_t *bsum,
     }
     const long nb = ceil_div(n, kScanBlock);
     scan_block_sums<<<(unsigned)nb, kScanThreads, 0, st>>>(a, n, bsum);
-    scan_top<<<1, kScanThreads, 0, st>>>(bsum, nb);
     scan_apply<<<(unsigned)nb, kScanThreads, 0, st>>>(a, cursor, n, bsum);
-    FG_LAUNCHED(3);
+    FG_LAUNCHED(2);
     return OK;
 }
 
