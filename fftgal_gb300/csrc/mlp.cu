@@ -173,6 +173,7 @@ mlp_grad_kernel(const float *__restrict__ params, const float *__restrict__ X, c
         b3[tid] = params[kOffB3 + tid];
         if (tid < kOut) b4[tid] = params[kOffB4 + tid];
     }
+    float part = 0.f;  // this lane's share of the loss
     for (long s0 = (long)blockIdx.x * kMlpS; s0 < n; s0 += (long)gridDim.x * kMlpS) {
         const int S = n - s0 < kMlpS ? (int)(n - s0) : kMlpS;
         __syncthreads();  // the parameters, or the previous round's reads
@@ -199,7 +200,6 @@ mlp_grad_kernel(const float *__restrict__ params, const float *__restrict__ X, c
         mlp_put(a3, z, lane, warp);
         __syncwarp();
         // outputs and their deltas: lane = (sample, output) of the warp's 12
-        float part = 0.f;
         if (lane < 4 * kOut) {
             const int q = 4 * warp + lane / kOut, o = lane % kOut;
             float y = b4[o];
@@ -207,12 +207,9 @@ mlp_grad_kernel(const float *__restrict__ params, const float *__restrict__ X, c
             for (int i = 0; i < kHid; ++i) y = fmaf(a3[i * kPitch + q], W4[i * kOut + o], y);
             float r = 0.f;
             if (q < S) r = y - T[(s0 + q) * kOut + o];
-            part = scale * r * r;
+            part += scale * r * r;
             dy[o * kPitch + q] = 2.f * scale * r;
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-        if (lane == 0) atomicAdd(loss, part);
         __syncwarp();
         mlp_back<kOut>(dy, W4, kOut, a3, d3, lane, warp);
         __syncwarp();
@@ -231,6 +228,17 @@ mlp_grad_kernel(const float *__restrict__ params, const float *__restrict__ X, c
                 g = i < kHid ? fmaf(a3[i * kPitch + q], dy[o * kPitch + q], g) : g + dy[o * kPitch + q];
             atomicAdd(i < kHid ? &grad[kOffW4 + e] : &grad[kOffB4 + o], g);
         }
+    }
+    // the loss: one addition to the caller's sum per CTA, as few roundings as there are CTAs
+    __shared__ float wsum[kMlpThreads / 32];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+    if (lane == 0) wsum[warp] = part;
+    __syncthreads();
+    if (tid == 0) {
+        float sum = 0.f;
+        for (int w = 0; w < kMlpThreads / 32; ++w) sum += wsum[w];
+        atomicAdd(loss, sum);
     }
 }
 
