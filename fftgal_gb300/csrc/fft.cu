@@ -519,17 +519,17 @@ static int scale_grids(const FftPlan *p, void *const *grids, int ngrids, double 
 }
 
 // The k pass: powers of two take fft2.cu's packed rows (half-length transforms);
-// other lengths the row pairs of fft3.cu where they split; the general kernels
-// below do the rest (c2r at Ng = 512: 733 us there, 518 in fft3.cu, 215 in fft2.cu;
-// both grids forward at Ng = 384: 1402 us there, 266 in fft3.cu).
+// other lengths fft3.cu's fused radix passes, which give the general kernels' results
+// (both grids forward at Ng = 384: 430 us against 1402); FP64 grids and lengths of a
+// single group of radices (or beyond fft3.cu's shared memory) the general kernels
+// below (c2r at Ng = 512: 733 us there, 215 in fft2.cu).
 static int k_pass(const FftPlan *p, void *const *grids, int ngrids, bool forward, cudaStream_t s, double scale = 1) {
     if (fft2_supported(p->Ng, p->prec)) {
         void *g1 = ngrids > 1 ? grids[1] : grids[0];
         return forward ? fft2_k_r2c(p->Ng, p->half.tw, p->rtw, grids[0], g1, ngrids, s, p->tune[0])
                        : fft2_k_c2r(p->Ng, p->half.tw, p->rtw, grids[0], g1, ngrids, scale, s);
     }
-    if (fft3_supported(p->Ng, p->prec))
-        return fft3_k(p->Ng, p->axis.tw, grids[0], ngrids > 1 ? grids[1] : grids[0], ngrids, forward, scale, s);
+    if (fft3_supported(p)) return fft3_k(p, grids[0], ngrids > 1 ? grids[1] : grids[0], ngrids, forward, scale, s);
     const long nrows = (long)p->Ng * p->Ng;
     const Fft1dPlan &kp = p->even ? p->half : p->axis;
     const Fft1dDev d = to_dev(kp);
@@ -564,9 +564,9 @@ static int cols_pass(const FftPlan *p, void *const *grids, int ngrids, int sign,
     if (fft2_supported(p->Ng, p->prec))
         return fft2_cols(p->Ng, p->axis.tw, grids[0], ngrids > 1 ? grids[1] : grids[0], ngrids, p->nh,
                          elem_stride, batch_stride, p->Ng, sign, s, logC, scale);
-    if (fft3_supported(p->Ng, p->prec))
-        return fft3_cols(p->Ng, p->axis.tw, grids[0], ngrids > 1 ? grids[1] : grids[0], ngrids, p->nh, elem_stride,
-                         batch_stride, p->Ng, sign, scale, s);
+    if (fft3_supported(p))
+        return fft3_cols(p, grids[0], ngrids > 1 ? grids[1] : grids[0], ngrids, elem_stride, batch_stride, sign, scale,
+                         s);
     const Fft1dDev d = to_dev(p->axis);
     const long ncb = ceil_div(p->nh, p->cols);
     dim3 grid((unsigned)(ncb * p->Ng), ngrids);

@@ -18,7 +18,7 @@
 // CTA pairs (fft2_cols1024_kernel), length 2048 is
 // 32 x 64 with the 64-point second step split over lane pairs
 // (fft2_cols2048_kernel).  Used for the k pass both ways (r2c, c2r) and the
-// strided j/i passes of FP32 grids; other lengths use fft3.cu's mixed-radix passes or,
+// strided j/i passes of FP32 grids; other lengths use fft3.cu's fused radix passes or,
 // where those do not apply (FP64 grids among them), the general kernels of fft.cu.
 #include "internal.h"
 #include "common.cuh"
@@ -426,8 +426,8 @@ fft2_k_r2c_kernel(float *g0, float *g1, long nrows, int Ng_pad, int R,
 // X[M-k] for each of its k = N2 n1 + n2 (the second reading of a row hits L1), so Z
 // needs no trip through shared memory; step 2 stores to the rows.  The imaginary
 // parts of X[0] and X[M] are ignored, and the row padding keeps its values, scaled
-// like the rest of the grid.  One grid of Ng = 512: 518 us with the row pairs of
-// fft3.cu (whole-length transforms, four trips through shared memory), about 215 here.
+// like the rest of the grid.  One grid of Ng = 512: 733 us in the general
+// kernels, about 215 here.
 template <int N1, int N2>
 __global__ void __launch_bounds__(512)
 fft2_k_c2r_kernel(float *g0, float *g1, long nrows, int Ng_pad, int R, const float2 *__restrict__ W,

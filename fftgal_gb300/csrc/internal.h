@@ -105,12 +105,12 @@ int fft2_prepare();
 bool fft2_tma_supported(int Ng, int prec);
 int fft2_cols_tma(int Ng, const void *W, void *g0, void *g1, int ngrids, int sign, cudaStream_t s);
 int fft2_tma_check();
-// mixed-radix FP32 passes (fft3.cu): Ng = N1 N2 with N1, N2 <= 32 and prime
-// factors up to 13; the k pass both ways (forward r2c, backward c2r)
-bool fft3_supported(int Ng, int prec);
-int fft3_cols(int N, const void *W, void *g0, void *g1, int ngrids, int ncols, long es, long bs, long nbatch, int sign,
-              double scale, cudaStream_t s);
-int fft3_k(int Ng, const void *W, void *g0, void *g1, int ngrids, bool forward, double scale, cudaStream_t s);
+// fused radix passes of FP32 grids (fft3.cu): a strided axis of the plan's grid, and
+// the k pass both ways (forward r2c, backward c2r)
+bool fft3_supported(const FftPlan *p);
+int fft3_cols(const FftPlan *p, void *g0, void *g1, int ngrids, long es, long bs, int sign, double scale,
+              cudaStream_t s);
+int fft3_k(const FftPlan *p, void *g0, void *g1, int ngrids, bool forward, double scale, cudaStream_t s);
 // time every valid launch shape of the three r2c passes on `grid` (one FP32
 // grid of the plan's size; its contents are transformed in place) and keep the
 // fastest in p->tune; ms[3] = the chosen shapes' times
@@ -140,9 +140,8 @@ struct PaintTiling {
     int tab_off[3] = {0, 0, 0};   // offset of axis a's tables in d_tables
     long nkeys = 0;               // nt0*nt1*nt2 * 27 (FP32 grids: 27 boundary classes) or * 1 (FP64)
     int cta_per_sm = 0;           // persistent FP32 tile-paint CTAs per SM (1 or 2; 0: built-in 2)
-    // tiles of up to 32 x 16 x 32 cells for FP32 paints of one grid (owned;
-    // null where Ng < 64): the one grid's accumulators fill the shared memory
-    // that two grids of 16 x 16 x 32 take
+    // FP32 grids with Ng >= 64: the tiles of up to 32 x 16 x 32 cells that their
+    // paints take, one grid per CTA (owned; null otherwise)
     PaintTiling *one = nullptr;
 };
 
