@@ -7,13 +7,13 @@
 //
 //  1. count   : every particle gets the key (tile, class) of its base cell.  The
 //               grid is cut into tiles of at most 32 x 16 x 32 cells (i, j, k;
-//               FP32 grids with Ng >= 64) or 16 x 16 x 32 (FP64, smaller Ng);
-//               per axis the class says whether the particle's stencil (over
+//               FP32 grids with Ng >= 64), 16 x 16 x 32 (smaller FP32 grids) or
+//               8 x 8 x 16 (FP64 grids, whose key is the tile alone); per axis the class says whether the particle's stencil (over
 //               all painted grids) reaches into the lower (1) or upper (2)
 //               neighbour tile, or neither (0).  Only the key histogram is
 //               written (fire-and-forget atomics).
-//  2. scan    : exclusive prefix sum of the key histogram, copied to a cursor
-//               array.
+//  2. scan    : exclusive prefix sum of the key histogram, written to a cursor
+//               array too.
 //  3. scatter : the key is formed again and each particle's record is written
 //               at the slot its key's cursor atomic returns.  The order within
 //               a key depends on the atomics' order; the FP32 paint sums in
@@ -47,8 +47,9 @@
 // many tiny products at a stencil's edge round to zero and bias the edge cells
 // low by several percent.  Integer sums are order independent, so the painted
 // grid is bit-reproducible run to run.
-// FP64 grids (paint_tile_f64_kernel) reproduce the reference's FP64 weight
-// arithmetic op for op and accumulate in FP64, one thread per particle.
+// FP64 grids (paint_warp_f64_kernel) reproduce the reference's FP64 weight
+// arithmetic op for op and accumulate in FP64: a warp owns a tile's cells and their
+// halo in shared memory and adds them to the zeroed grid.
 #include "internal.h"
 #include "common.cuh"
 
