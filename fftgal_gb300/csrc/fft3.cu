@@ -297,8 +297,8 @@ __device__ __forceinline__ void run_group(int code, const GroupArgs &g) {
 // global memory or, with p null, a buffer; the offset of the last one used is
 // returned, and the caller synchronises before reading it.
 template <bool COLS>
-__device__ __forceinline__ int fft_groups(const Groups &f, const Side &src, const Side &dst, const Side &buf, int other, int ncol,
-                          int logc, int sign, float scale) {
+__device__ __forceinline__ int fft_groups(const Groups &f, const Side &src, const Side &dst, const Side &buf,
+                                          int other, int ncol, int logc, int sign, float scale) {
     GroupArgs g;
     g.W = f.W;
     g.n = f.n;
