@@ -8,9 +8,10 @@
 //  1. count   : every particle gets the key (tile, class) of its base cell.  The
 //               grid is cut into tiles of at most 32 x 16 x 32 cells (i, j, k;
 //               FP32 grids with Ng >= 64), 16 x 16 x 32 (smaller FP32 grids) or
-//               8 x 8 x 16 (FP64 grids, whose key is the tile alone); per axis the class says whether the particle's stencil (over
-//               all painted grids) reaches into the lower (1) or upper (2)
-//               neighbour tile, or neither (0).  Only the key histogram is
+//               8 x 8 x 16 (FP64 grids, whose key is the tile alone); per axis
+//               the class says whether the particle's stencil (over all painted
+//               grids) reaches into the lower (1) or upper (2) neighbour tile, or
+//               neither (0).  Only the key histogram is
 //               written (fire-and-forget atomics).
 //  2. scan    : exclusive prefix sum of the key histogram, written to a cursor
 //               array too.
