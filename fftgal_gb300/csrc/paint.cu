@@ -718,9 +718,12 @@ __device__ __forceinline__ int tile_fixbits(uint32_t total, const uint4 *__restr
             if (cyc[a]) {
                 bb = b / kBlk;
             } else {
+                // a tile's particles have their base cells at -3 .. te + 1 (te <= Ng - 6), and
+                // images are folded there as record_axis does: with two tiles along an
+                // axis te and te + 1 are half a box away or more
                 int l = b - ts.t0[a];
-                if (l > Ng / 2) l -= Ng;
-                if (l < -Ng / 2) l += Ng;
+                l += l < -4 ? Ng : 0;
+                l -= l >= Ng - 4 ? Ng : 0;
                 bb = (l + 4) / kBlk;  // margin of 4 cells below the tile
                 bb = bb < 0 ? 0 : (bb >= nb[a] ? nb[a] - 1 : bb);
             }
