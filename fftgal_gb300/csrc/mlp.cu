@@ -179,7 +179,9 @@ mlp_grad_kernel(const float *__restrict__ params, const float *__restrict__ X, c
         __syncthreads();  // the parameters, or the previous round's reads
         for (int e = tid; e < kMlpS * kIn; e += kMlpThreads) {
             const int q = e / kIn, i = e - q * kIn;
-            x0[i * kPitch + q] = q < S ? X[s0 * kIn + e] : 0.f;
+            // beyond the last sample its copies, whose output deltas are 0: values of their
+            // own could make 0 x inf = NaN of a weight that is infinite
+            x0[i * kPitch + q] = X[q < S ? s0 * kIn + e : (n - 1) * kIn + i];
         }
         __syncthreads();
         float z[2][4];
