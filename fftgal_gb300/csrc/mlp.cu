@@ -257,41 +257,69 @@ __global__ void mlp_adam_kernel(float *__restrict__ params, const float *__restr
     params[e] -= lr * (mm / c1) / (sqrtf(vv / c2) + eps);
 }
 
-// y = f(x): a warp per sample, lane l the hidden units l and l + 32, the sums over
-// the inputs in ascending order.  The learned call at Ng = 256 (222 bins, 56 CTAs):
-// 536 -> 467 us against one thread per sample (two CTAs, the activations in local
-// memory: 67 us the kernel).
+// y = f(x): a warp takes NS samples at a time, lane l the hidden units l and l + 32, the
+// sums over the inputs in ascending order.  NS = 1 where there are few samples: the
+// learned call at Ng = 256 (222 bins, 56 CTAs) 536 -> 467 us against one thread per
+// sample (two CTAs, the activations in local memory: 67 us the kernel).  NS = 4 shares
+// the two weights that a lane reads per input among four samples, from as many samples
+// as give every warp four: 2e4 samples 54 -> 31 us, 7e5 1311 -> 450 (a thread per sample:
+// 74 and 691).
 constexpr int kFwdWarps = 4;
+template <int NS> struct __align__(4 * NS) Samples {
+    float v[NS];
+};
+template <int NS>
 __global__ void __launch_bounds__(32 * kFwdWarps)
 mlp_forward_kernel(const float *__restrict__ params, const float *__restrict__ X, long n, float *__restrict__ Y) {
     __shared__ __align__(16) float P[kNParams];
-    __shared__ float act[kFwdWarps][2][kHid];
+    __shared__ Samples<NS> act[kFwdWarps][2][kHid];
     for (int e = threadIdx.x; e < kNParams; e += blockDim.x) P[e] = params[e];
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float *a = act[warp][0], *b = act[warp][1];
-    for (long s = blockIdx.x * (long)kFwdWarps + warp; s < n; s += (long)gridDim.x * kFwdWarps) {
-        auto dense = [&](const float *x, int nin, int oW, int ob, float *out) {
-            float z0 = P[ob + lane], z1 = P[ob + lane + 32];
+    Samples<NS> *a = act[warp][0], *b = act[warp][1];
+    const long step = (long)gridDim.x * kFwdWarps * NS;
+    for (long s = (blockIdx.x * (long)kFwdWarps + warp) * NS; s < n; s += step) {
+        auto dense = [&](const Samples<NS> *x, int nin, int oW, int ob, Samples<NS> *out) {
+            Samples<NS> z0, z1;
+#pragma unroll
+            for (int q = 0; q < NS; ++q) {
+                z0.v[q] = P[ob + lane];
+                z1.v[q] = P[ob + lane + 32];
+            }
 #pragma unroll 8
             for (int i = 0; i < nin; ++i) {
-                z0 = fmaf(x[i], P[oW + i * kHid + lane], z0);
-                z1 = fmaf(x[i], P[oW + i * kHid + lane + 32], z1);
+                const float w0 = P[oW + i * kHid + lane], w1 = P[oW + i * kHid + lane + 32];
+                const Samples<NS> u = x[i];
+#pragma unroll
+                for (int q = 0; q < NS; ++q) {
+                    z0.v[q] = fmaf(u.v[q], w0, z0.v[q]);
+                    z1.v[q] = fmaf(u.v[q], w1, z1.v[q]);
+                }
             }
-            out[lane] = tanhf(z0);
-            out[lane + 32] = tanhf(z1);
+#pragma unroll
+            for (int q = 0; q < NS; ++q) {
+                z0.v[q] = tanhf(z0.v[q]);
+                z1.v[q] = tanhf(z1.v[q]);
+            }
+            out[lane] = z0;
+            out[lane + 32] = z1;
             __syncwarp();
         };
-        if (lane < kIn) b[lane] = X[s * kIn + lane];
+        const int S = n - s < NS ? (int)(n - s) : NS;
+        if (lane < kIn * NS) {
+            const int q = lane / kIn, i = lane - q * kIn;
+            b[i].v[q] = X[(s + (q < S ? q : S - 1)) * kIn + i];
+        }
         __syncwarp();
         dense(b, kIn, kOffW1, kOffB1, a);
         dense(a, kHid, kOffW2, kOffB2, b);
         dense(b, kHid, kOffW3, kOffB3, a);
-        if (lane < kOut) {
-            float z = P[kOffB4 + lane];
+        if (lane < kOut * S) {
+            const int q = lane / kOut, o = lane - q * kOut;
+            float z = P[kOffB4 + o];
 #pragma unroll 8
-            for (int i = 0; i < kHid; ++i) z = fmaf(a[i], P[kOffW4 + i * kOut + lane], z);
-            Y[s * kOut + lane] = z;
+            for (int i = 0; i < kHid; ++i) z = fmaf(a[i].v[q], P[kOffW4 + i * kOut + o], z);
+            Y[(s + q) * kOut + o] = z;
         }
         __syncwarp();
     }
@@ -335,9 +363,15 @@ extern "C" int fftgal_mlp_adam(float *params, const float *grad, float *m, float
 
 extern "C" int fftgal_mlp_forward(const float *params, const float *X, long n, float *Y, void *stream) {
     if (!params || !X || !Y || n < 1) return set_error(ERR_ARG, "fftgal_mlp_forward: bad arguments");
-    long nb = ceil_div(n, kFwdWarps);
+    const long full = 4L * num_sms() * kFwdWarps;  // warps of a full grid
+    const int ns = n >= 4 * full ? 4 : 1;
+    long nb = ceil_div(n, kFwdWarps * ns);
     if (nb > 4L * num_sms()) nb = 4L * num_sms();
-    mlp_forward_kernel<<<(unsigned)nb, 32 * kFwdWarps, 0, static_cast<cudaStream_t>(stream)>>>(params, X, n, Y);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (ns == 4)
+        mlp_forward_kernel<4><<<(unsigned)nb, 32 * kFwdWarps, 0, st>>>(params, X, n, Y);
+    else
+        mlp_forward_kernel<1><<<(unsigned)nb, 32 * kFwdWarps, 0, st>>>(params, X, n, Y);
     FG_LAUNCHED(1);
     return OK;
 }
