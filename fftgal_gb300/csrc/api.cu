@@ -422,7 +422,7 @@ static std::map<std::tuple<int, int, int>, LaunchTune> g_launch_cache;
 // The counterpart of plan_resolve for the paint and binning launch shapes of
 // an FP32 grid with the two-level FFT: the plan file's launch line for this
 // device and Ng, else this process's earlier measurement, else timing every
-// shape (binning: 1-3 CTAs per SM x fold every 8 or 32 blocks on zero grids;
+// shape (binning: up to 3 CTAs per SM x fold every 8 or 32 blocks on zero grids;
 // tile paint: 1 or 2 persistent CTAs per SM on a uniform catalog of Ng^3/10
 // particles) and writing the line.  The built-in shape stays unless another
 // is more than 2 % faster.  The grids are left zeroed.
@@ -469,15 +469,16 @@ static int tune_launch(fft_t *self, const char *path) {
             fin.w32 = winv_tab32(g);
             fin.scale = 0.5 * H3_of(g);
             double best_b = 0, def_b = 0;
-            t.bin_cta = 3;
+            const int most = bin_cta_builtin(bs, 5);  // more are the same launch
+            t.bin_cta = most;
             t.bin_fold = 8;
-            for (int cta = 3; cta >= 1; --cta)
+            for (int cta = most; cta >= 1; --cta)
                 for (int fold : {8, 32}) {
                     geo->cta_per_sm = cta;
                     geo->fold = fold;
                     double ms = 0;
                     FG_TRY(median_ms(st, [&]() { return bin_power_launch(geo, 5, 1.0, 0.0, st, &fin, nullptr); }, &ms));
-                    if (cta == 3 && fold == 8) {
+                    if (cta == most && fold == 8) {
                         def_b = best_b = ms;
                     } else if (ms < best_b && ms < 0.98 * def_b) {
                         best_b = ms;
@@ -1115,7 +1116,11 @@ extern "C" int fftgal_launch_shapes(fft_t *grid, int shapes[3], int *source, dou
     Grid *g = G(grid);
     if (shapes) {
         shapes[0] = g->launch.paint_cta > 0 ? g->launch.paint_cta : 2;
-        shapes[1] = g->launch.bin_cta > 0 ? g->launch.bin_cta : 3;
+        const double los[3] = {0, 0, 1};
+        BinSpec bs;
+        FG_TRY(bin_spec_init(&bs, grid->Ng, grid->L, 2 * M_PI / grid->L, los, 3));
+        const int most = g->prec == 4 ? bin_cta_builtin(bs, 5) : 3;
+        shapes[1] = g->launch.bin_cta > 0 && g->launch.bin_cta < most ? g->launch.bin_cta : most;
         shapes[2] = g->launch.bin_fold > 0 ? g->launch.bin_fold : 0;
     }
     if (source) *source = g->launch_source;

@@ -358,6 +358,11 @@ static SlabMirror slab_mirror(const BinSpec &s) {
     return m;
 }
 
+// the kernels whose CTAs per SM a measured launch shape sets: it is measured on both
+// interlacing grids with the line of sight along z, and the kernels of one grid, or of
+// fewer mirrored modes, have an optimum of their own
+static bool tuned_slab(int np, int mode) { return np == 4 && (mode == 2 || mode == 5); }
+
 // The slab blocks cover k < kmain.  When the half spectrum's last k block
 // would hold only one or two columns (nh = Ng/2 + 1: the Nyquist column of
 // every even Ng that is a multiple of 32), those columns are binned mode by
@@ -603,6 +608,40 @@ static size_t slab_smem(int NK, int NQ, int warps = kSlabThreads / 32) {
            sizeof(float) * warps * kSlabJ * kSlabRow;
 }
 
+// the launch of the slab kernel: mirrored modes, rows of a slab, warps of a CTA, slabs,
+// CTAs per SM, shared memory
+struct SlabShape {
+    SlabMirror mir;
+    int np = 1, nr = kSlabJ, warps = kSlabThreads / 32, per_sm = 1;
+    long units = 0;
+    size_t smem = 0;
+};
+
+static SlabShape slab_shape(const BinSpec &s, int mode) {
+    SlabShape h;
+    h.mir = slab_mirror(s);
+    h.np = h.mir.modes();
+    // small grids: shorter slabs until there are 16 warps' worth per SM, and
+    // smaller CTAs until there are two per SM
+    const long blocks = ceil_div(h.mir.NI, kSlabI) * ceil_div(h.mir.NJ, kSlabJ) *
+                        ceil_div(slab_kmain(s.Ng / 2 + 1), kSlabK);
+    while (h.nr > 4 && blocks * kSlabI * (kSlabJ / h.nr) < 16L * num_sms()) h.nr /= 2;
+    h.units = blocks * kSlabI * (kSlabJ / h.nr);
+    while (h.warps > 4 && h.units / h.warps < 2L * num_sms()) h.warps /= 2;
+    h.smem = slab_smem(s.NK, 4 + s.Nmu + 1, h.warps);
+    const int per_sm = (int)((224 * 1024) / (h.smem + 1024));
+    // three CTAs per SM hide the loads best, except where four mirrored modes of
+    // two grids want 16 loads in flight and the grid is large: two CTAs without
+    // spills (interlaced, los along z: Ng = 1024 1.94 against 2.27 ms, 512 305 against
+    // 348 us, 384 158 against 180, but 256 84 against 76, 128 28.7 against 24.6; two
+    // mirrored modes at 512 524 against 479 us)
+    const int most = tuned_slab(h.np, mode) && h.units >= 64L * num_sms() ? 2 : 3;
+    h.per_sm = per_sm < 1 ? 1 : (per_sm > most ? most : per_sm);
+    return h;
+}
+
+int bin_cta_builtin(const BinSpec &s, int mode) { return slab_shape(s, mode).per_sm; }
+
 static int bin_launch(BinGeometry *g, const void *f, int prec, int mode, double Vinv, double Pshot, cudaStream_t st,
                       const BinFinish *fin, const DevScalars *ds);
 
@@ -643,28 +682,13 @@ static int bin_launch(BinGeometry *g, const void *f, int prec, int mode, double 
         return set_error(ERR_UNSUPPORTED, "binning: %d k bins x %d wedges exceed shared memory", NK, s.Nmu);
     FG_CUDA(cudaMemsetAsync(g->d_acc, 0, sizeof(double) * g->acc_len, st));
     if (prec == 4) {
-        const SlabMirror mir = slab_mirror(s);
-        const int np = mir.modes();
-        // small grids: shorter slabs until there are 16 warps' worth per SM, and
-        // smaller CTAs until there are two per SM
-        const long blocks = ceil_div(mir.NI, kSlabI) * ceil_div(mir.NJ, kSlabJ) *
-                            ceil_div(slab_kmain(s.Ng / 2 + 1), kSlabK);
-        int nr = kSlabJ;
-        while (nr > 4 && blocks * kSlabI * (kSlabJ / nr) < 16L * num_sms()) nr /= 2;
-        const long units = blocks * kSlabI * (kSlabJ / nr);
-        int warps = kSlabThreads / 32;
-        while (warps > 4 && units / warps < 2L * num_sms()) warps /= 2;
-        smem = slab_smem(NK, NQ, warps);
-        int per_sm = (int)((224 * 1024) / (smem + 1024));
-        // three CTAs per SM hide the loads best, except where four mirrored modes of
-        // two grids want 16 loads in flight and the grid is large: two CTAs without
-        // spills (interlaced, los along z: Ng = 1024 1.94 against 2.27 ms, 512 305 against
-        // 348 us, 384 158 against 180, but 256 84 against 76, 128 28.7 against 24.6; two
-        // mirrored modes at 512 524 against 479 us)
-        const bool two = np == 4 && (mode == 2 || mode == 5) && units >= 64L * num_sms();
-        per_sm = per_sm < 1 ? 1 : (per_sm > (two ? 2 : 3) ? (two ? 2 : 3) : per_sm);
-        if (g->cta_per_sm > 0 && g->cta_per_sm < per_sm) per_sm = g->cta_per_sm;  // tuned shape
-        const long nturn = units / warps;
+        const SlabShape h = slab_shape(s, mode);
+        const SlabMirror mir = h.mir;
+        const int np = h.np, nr = h.nr, warps = h.warps;
+        smem = h.smem;
+        int per_sm = h.per_sm;
+        if (tuned_slab(np, mode) && g->cta_per_sm > 0 && g->cta_per_sm < per_sm) per_sm = g->cta_per_sm;
+        const long nturn = h.units / warps;
         long nb = (long)num_sms() * per_sm;
         if (nb > nturn) nb = nturn;
         SlabFinish sf;

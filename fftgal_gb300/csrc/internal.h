@@ -240,7 +240,8 @@ struct BinGeometry {               // data-independent part, cached
     double *d_acc = nullptr;      // device accumulators (per call)
     size_t acc_len = 0;
     int bad = 0;
-    // FP32 binning launch shape (0: built-in): CTAs per SM, blocks between folds
+    // FP32 binning launch shape (0: built-in): CTAs per SM of the interlaced finish with
+    // four mirrored modes, blocks between folds
     int cta_per_sm = 0, fold = 0;
 };
 
@@ -272,6 +273,8 @@ int bin_power(BinGeometry *g, const void *f, int prec, int mode, double Vinv, do
 // takes Vinv and Pshot from device memory
 int bin_power_launch(BinGeometry *g, int mode, double Vinv, double Pshot, cudaStream_t st, const BinFinish *fin,
                      const DevScalars *ds);
+// CTAs per SM of the built-in launch of FP32 `mode`
+int bin_cta_builtin(const BinSpec &s, int mode);
 // Psum / Pw of bin_power from a copy of g->d_acc
 void bin_power_unpack(const BinGeometry *g, const double *acc, double *Psum, double *Pw);
 

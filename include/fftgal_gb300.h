@@ -216,9 +216,11 @@ int fftgal_plan_info(fft_t *grid, int tune[3], int *source, double ms[3]);
 int fftgal_plan_autotune(fft_t *grid, double ms[3]);
 /* Launch shapes of the tile paint and of the finish + binning kernel of an
  * FP32 grid (power-of-two Ng): shapes[0] = persistent paint CTAs per SM
- * (1 or 2), shapes[1] = binning CTAs per SM (1-3, fewer when its shared
- * accumulators do not fit), shapes[2] = binning blocks between the folds of
- * its FP32 sums into FP64 (0: built-in, 8 or FFTGAL_BIN_FOLD).  With a plan
+ * (1 or 2), shapes[1] = CTAs per SM of the binning that finishes both
+ * interlacing grids with a line of sight along an axis (1-3, at Ng, Nmu = 3 and
+ * bins of 2 pi / L; other binning kernels keep their built-in shapes), shapes[2]
+ * = binning blocks between the folds of the FP32 sums into FP64 (0: built-in,
+ * 8 or FFTGAL_BIN_FOLD).  With a plan
  * file, fft_init imports them from the file's "fftgal_gb300-launch" line for
  * this device and Ng, or times every shape (binning on zero grids, the paint
  * on a uniform catalog of Ng^3/10 particles; built-in kept unless another is
