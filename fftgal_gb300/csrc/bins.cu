@@ -429,12 +429,13 @@ __device__ __forceinline__ void bin_single(const BinDev &d, const SlabFinish &fi
 // nr: rows of a slab and modes of a run, 16 or, on small grids, 8 or 4, so that
 // a block makes 16 x 16 / nr slabs for as many warps (a warp takes 20 us or more
 // for 16 rows, whatever the grid; the CTA's blockDim.x / 32 warps take as many
-// slabs of a block per turn).
-template <int MODE, int NP, int MINB>
+// slabs of a block per turn).  FULL: 16 rows and 16 warps, known to the compiler, for
+// the one-mode slabs, whose row loop is most of their work.
+template <int MODE, int NP, int MINB, bool FULL>
 __global__ void __launch_bounds__(kSlabThreads, MINB)
 bin_power_slab_kernel(BinDev d, const float2 *__restrict__ f, SlabFinish fin, SlabMirror mir, float Vinv, float Pshot,
                       const uint32_t *__restrict__ thr_g, double *__restrict__ gacc, const DevScalars *__restrict__ ds,
-                      int fold, int nr) {
+                      int fold, int nr_) {
     if (ds) {
         Vinv = ds->Vinv;
         Pshot = ds->Pshot;
@@ -444,12 +445,13 @@ bin_power_slab_kernel(BinDev d, const float2 *__restrict__ f, SlabFinish fin, Sl
     float *acc32 = reinterpret_cast<float *>(smem_raw);                        // [NQ][NK]
     uint32_t *thr = reinterpret_cast<uint32_t *>(acc32 + (size_t)NK * NQ);     // [NK + 2]
     float *slabs = reinterpret_cast<float *>(thr + ((NK + 2 + 3) & ~3));        // [warps][16][kSlabRow]
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = FULL ? kSlabThreads / 32 : blockDim.x >> 5;
+    const int nr = FULL ? kSlabJ : nr_;
     float *slab = slabs + warp * kSlabJ * kSlabRow;
     for (int e = tid; e < NK * NQ; e += blockDim.x) acc32[e] = 0.f;
     for (int e = tid; e < NK + 2; e += blockDim.x) thr[e] = thr_g[e];
     __syncthreads();
-    const int Ng = d.Ng, nh = d.nh, kmain = slab_kmain(nh), NI = mir.NI, NJ = mir.NJ;
+    const int Ng = d.Ng, nh = d.nh, kmain = slab_kmain(nh), NI = NP == 1 ? d.Ng : mir.NI, NJ = NP == 1 ? d.Ng : mir.NJ;
     const int nbi = (NI + kSlabI - 1) / kSlabI, nbj = (NJ + kSlabJ - 1) / kSlabJ, nbk = (kmain + kSlabK - 1) / kSlabK;
     const int nsub = kSlabI * (kSlabJ / nr) / nwarp;  // CTA turns per block
     const int nblk = nbi * nbj * nbk * nsub;
@@ -498,10 +500,11 @@ bin_power_slab_kernel(BinDev d, const float2 *__restrict__ f, SlabFinish fin, Sl
             const long rs = rows_i ? si : sj, fs = rows_i ? sj : si;
             const float2 *fk = f;
             const long eF = fixed * fs + k, eG = (cf ? fm : fixed) * fs + k;
+            long en = r0 * rs + eF;
             // unrolled for 8 or 16 loads in flight, as far as the registers go
             constexpr int UNR = MINB >= 3 ? (NP == 1 ? 8 : 4 / NP) : (NP == 1 ? 8 : 8 / NP);
 #pragma unroll UNR
-            for (int r = 0; r < nr; ++r) {
+            for (int r = 0; r < nr; ++r, en += rs) {
                 float2 pr = make_float2(0.f, 0.f);
                 float wr = 0.f;
                 if (MODE == 2 || MODE == 5) {
@@ -513,10 +516,23 @@ bin_power_slab_kernel(BinDev d, const float2 *__restrict__ f, SlabFinish fin, Sl
                 const int x = r0 + r;
                 if (x < nrow && k < kmain) {
                     const float wk = wfk * wr;
-                    const long e0 = x * rs + eF;
+                    const long e0 = NP == 1 ? en : x * rs + eF;
                     if (NP == 1) {
-                        const float s = mode_value<MODE>(fin, mode_load<MODE>(fin, fk, e0), e0, cmul(q0, pr), wk, true);
-                        pv = mode_power<MODE>(s, 1.f, wk, Vinv, Pshot);
+                        // one mode per element: with the same arithmetic as below, written as
+                        // its own product, the compiler keeps eight pairs of loads in flight
+                        // (los (1, 1, 1), Ng = 1024, interlaced 5.02 -> 4.48 ms, with FULL and
+                        // the running index, which also take single paints from 4.15 to 3.77)
+                        if (MODE == 2 || MODE == 5) {
+                            const float2 p = cmul(q0, pr);
+                            const float2 bv = fin.B[e0], av = fin.A[e0];
+                            const float2 dv = cmul(bv, p);
+                            const float2 v = make_float2((dv.x + av.x) * wk, (dv.y + av.y) * wk);
+                            if (MODE == 2) fin.A[e0] = v;
+                            pv = (v.x * v.x + v.y * v.y) * Vinv - Pshot;
+                        } else {
+                            const float s = mode_value<MODE>(fin, mode_load<MODE>(fin, fk, e0), e0, q0, wk, true);
+                            pv = mode_power<MODE>(s, 1.f, wk, Vinv, Pshot);
+                        }
                     } else {
                         const bool has_r = x > 0 && 2 * x != Ng;
                         const long xm = x ? Ng - x : 0;
@@ -625,18 +641,32 @@ static SlabShape slab_shape(const BinSpec &s, int mode) {
     // smaller CTAs until there are two per SM
     const long blocks = ceil_div(h.mir.NI, kSlabI) * ceil_div(h.mir.NJ, kSlabJ) *
                         ceil_div(slab_kmain(s.Ng / 2 + 1), kSlabK);
-    while (h.nr > 4 && blocks * kSlabI * (kSlabJ / h.nr) < 16L * num_sms()) h.nr /= 2;
-    h.units = blocks * kSlabI * (kSlabJ / h.nr);
-    while (h.warps > 4 && h.units / h.warps < 2L * num_sms()) h.warps /= 2;
-    h.smem = slab_smem(s.NK, 4 + s.Nmu + 1, h.warps);
-    const int per_sm = (int)((224 * 1024) / (h.smem + 1024));
     // three CTAs per SM hide the loads best, except where four mirrored modes of
     // two grids want 16 loads in flight and the grid is large: two CTAs without
     // spills (interlaced, los along z: Ng = 1024 1.94 against 2.27 ms, 512 305 against
     // 348 us, 384 158 against 180, but 256 84 against 76, 128 28.7 against 24.6; two
     // mirrored modes at 512 524 against 479 us)
-    const int most = tuned_slab(h.np, mode) && h.units >= 64L * num_sms() ? 2 : 3;
-    h.per_sm = per_sm < 1 ? 1 : (per_sm > most ? most : per_sm);
+    const int most = tuned_slab(h.np, mode) && blocks * kSlabI >= 64L * num_sms() ? 2 : 3;
+    auto fill = [&](int nr) {  // slabs of nr rows; returns the rows that a warp takes one after the other
+        h.nr = nr;
+        h.units = blocks * kSlabI * (kSlabJ / nr);
+        h.warps = kSlabThreads / 32;
+        while (h.warps > 4 && h.units / h.warps < 2L * num_sms()) h.warps /= 2;
+        h.smem = slab_smem(s.NK, 4 + s.Nmu + 1, h.warps);
+        const int per_sm = (int)((224 * 1024) / (h.smem + 1024));
+        h.per_sm = per_sm < 1 ? 1 : (per_sm > most ? most : per_sm);
+        return ceil_div(h.units / h.warps, (long)num_sms() * h.per_sm) * nr;
+    };
+    int nr = kSlabJ;
+    while (nr > 4 && blocks * kSlabI * (kSlabJ / nr) < 16L * num_sms()) nr /= 2;
+    // with few rounds of CTAs a last one of few takes as long as a full one: shorter
+    // slabs where that leaves an eighth fewer rows to do one after the other (interlaced,
+    // los (1, 1, 1): Ng = 144 61 -> 39 us; (1, 1, 0): 192 76 -> 53; z: 240 100 -> 55.
+    // With more rounds the shorter slabs' own cost counts: (1, 1, 1), 448 455 against 399)
+    long rows = fill(nr);
+    if (rows <= 3 * nr)
+        for (long r; nr > 4 && 8 * (r = fill(nr / 2)) <= 7 * rows; rows = r) nr /= 2;
+    fill(nr);
     return h;
 }
 
@@ -689,6 +719,7 @@ static int bin_launch(BinGeometry *g, const void *f, int prec, int mode, double 
         int per_sm = h.per_sm;
         if (tuned_slab(np, mode) && g->cta_per_sm > 0 && g->cta_per_sm < per_sm) per_sm = g->cta_per_sm;
         const long nturn = h.units / warps;
+        const bool full = nr == kSlabJ && warps == kSlabThreads / 32;
         long nb = (long)num_sms() * per_sm;
         if (nb > nturn) nb = nturn;
         SlabFinish sf;
@@ -700,22 +731,24 @@ static int bin_launch(BinGeometry *g, const void *f, int prec, int mode, double 
             sf.scale = (float)fin->scale;
         }
         const float2 *fv = static_cast<const float2 *>(mode >= 2 ? fin->A : f);
-#define FG_SLAB_LAUNCH3(M, N, B)                                                                             \
+#define FG_SLAB_LAUNCH3(M, N, B, F)                                                                          \
     do {                                                                                                    \
-        FG_CUDA(cudaFuncSetAttribute(bin_power_slab_kernel<M, N, B>,                                         \
+        FG_CUDA(cudaFuncSetAttribute(bin_power_slab_kernel<M, N, B, F>,                                      \
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));               \
-        bin_power_slab_kernel<M, N, B><<<(unsigned)nb, 32 * warps, smem, st>>>(                              \
+        bin_power_slab_kernel<M, N, B, F><<<(unsigned)nb, 32 * warps, smem, st>>>(                              \
             d, fv, sf, mir, (float)Vinv, (float)Pshot, g->d_thr, g->d_acc, ds,                               \
             g->fold > 0 ? g->fold : fold_blocks(), nr);                                                      \
     } while (0)
-#define FG_SLAB_LAUNCH2(M, B)            \
-    do {                                 \
-        if (np == 4)                     \
-            FG_SLAB_LAUNCH3(M, 4, B);    \
-        else if (np == 2)                \
-            FG_SLAB_LAUNCH3(M, 2, B);    \
-        else                             \
-            FG_SLAB_LAUNCH3(M, 1, B);    \
+#define FG_SLAB_LAUNCH2(M, B)                \
+    do {                                     \
+        if (np == 4)                         \
+            FG_SLAB_LAUNCH3(M, 4, B, false); \
+        else if (np == 2)                    \
+            FG_SLAB_LAUNCH3(M, 2, B, false); \
+        else if (full)                       \
+            FG_SLAB_LAUNCH3(M, 1, B, true);  \
+        else                                 \
+            FG_SLAB_LAUNCH3(M, 1, B, false); \
     } while (0)
 #define FG_SLAB_LAUNCH(M)             \
     do {                              \
