@@ -946,8 +946,8 @@ static int parity_tensor_map(CUtensorMap *tm, void *grid, int Ng) {
 
 bool fft2_tma_supported(int Ng, int prec) {
     // off by default: with 64-byte rows at the plane stride the TMA pass
-    // measured 7.8 ms against 4.7 ms for fft2_cols_kernel (16 columns, 128-byte
-    // rows) at Ng = 1024; FFTGAL_TMA=1 selects it
+    // measured 7.8 ms at Ng = 1024 against 4.7 of a pass of 16 columns per CTA
+    // (128-byte rows), which today's CTA pairs do in 3.6; FFTGAL_TMA=1 selects it
     static const int on = [] {
         const char *e = getenv("FFTGAL_TMA");
         return e && e[0] == '1';

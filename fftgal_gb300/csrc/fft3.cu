@@ -6,12 +6,15 @@
 // r Ns.  Up to three consecutive passes R1, R2, R3 (product M <= 32) need no memory in
 // between: a thread that holds the M values a + r3 N/M + r2 N/(R1 R2) + r1 N/R1
 // (a < N/M) has every butterfly of the three passes that its values meet.  So a
-// length is cut into two or three groups of passes, e.g. 384 = (8)(8 2)(3), 225 =
-// (3 3)(5 5): a thread loads a group's values (the first group from global memory,
-// the others from shared), transforms them in registers and stores them (the last
-// group to global memory).  The arithmetic, twiddle tables and order of operations
-// are the general kernels', and so are the results, bit for bit.  (A two-step form
-// with its own factors, N = N1 N2 in registers around one trip through shared memory, is
+// length is cut into two groups of passes or more, the fewest and then those with the
+// smallest largest one, e.g. 384 = (8)(8)(2 3), 225 = (3 3)(5 5): a thread loads a
+// group's values (the first group from global memory, the others from shared),
+// transforms them in registers and stores them (the last group to global memory).
+// The arithmetic, twiddle tables and order of operations are the general kernels'.
+// So are the results, bit for bit, with nvcc 13.0 (compared at 92 lengths): the
+// butterflies leave the fusing of products to the compiler in both files, so another
+// compiler may round them differently, which nothing relies on.  (A two-step form with
+// its own factors, N = N1 N2 in registers around one trip through shared memory, is
 // faster -- 384: 266 and 404 us for the passes below -- and its L2 error is no larger,
 // but the power of a small grid is dominated by a few modes at the cube's corner,
 // whose error then goes either way by up to 2.)
@@ -66,7 +69,7 @@ struct DftTable {
 __constant__ DftTable c_dft3 = DftTable();
 
 // The butterflies of fft.cu's general kernels, for FP32.  The sign stays a run-time
-// value as there: the compiler fuses the same products, so the results are the same.
+// value as there, so that the compiler fuses the same products.
 __device__ __forceinline__ void dft4(float2 &v0, float2 &v1, float2 &v2, float2 &v3, int sign) {
     const float2 a = cadd(v0, v2), b = csub(v0, v2);
     const float2 c = cadd(v1, v3), d = cmul_si(csub(v1, v3), sign);
@@ -503,7 +506,8 @@ static int buffers(const Groups &f, int q0, int q1, int ncol) {
 constexpr size_t kF3Smem = 100 * 1024;  // two CTAs per SM
 
 // columns per CTA: 8, 16 or 32 (64- to 256-byte rows), whatever costs least per column
-// with room for two CTAs
+// with room for two CTAs; where not even 8 columns fit (some lengths from 810 on, all
+// above 864) 4 or 2, whose rows of 32 or 16 bytes waste a part of each line
 static bool cols_shape(const Groups &f, int *logc, size_t *smem) {
     long best = 0;
     *logc = -1;

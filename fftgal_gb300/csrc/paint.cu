@@ -19,10 +19,12 @@
 //               at the slot its key's cursor atomic returns.  The order within
 //               a key depends on the atomics' order; the FP32 paint sums in
 //               fixed point, so the painted grid does not.
-//  4. paint   : one CTA per tile owns its cells.  It pulls the particles of its
-//               own tile and only the boundary classes of its 26 neighbours,
+//  4. paint   : FP32 grids: one CTA per tile owns its cells.  It pulls the particles
+//               of its own tile and only the boundary classes of its 26 neighbours,
 //               accumulates their weights in shared memory and writes every
 //               owned cell exactly once (no global atomics, no zeroing pass).
+//               FP64 grids: the grid is zeroed, and a warp adds the weights of its
+//               tile's own particles, halo included, with global atomics.
 //
 // FP32 grids with Ng >= 64 (paint_rot_kernel, persistent over tiles of
 // 32 x 16 x 32 cells, two 512-thread CTAs per SM): one thread deposits one
@@ -1093,7 +1095,7 @@ paint_coop_kernel(PaintParams pp, const uint32_t *__restrict__ off, const uint4 
 // Cells outside the tile: along i two blocks on either side of the sums take
 // them and along k one more block (of both sides), none of which is read; along
 // j they get weight 0 and the block 0 cell of their digit.  A dense tile paints
-// 16 rows at a time into 64-bit sums of the same layout.
+// 16 rows at a time into 64-bit sums of the same layout (rot_deposit_wide).
 // Bound by instruction issue (67 % of the slots at Ng = 512) and the barriers
 // between a tile's phases; 54 instructions per particle for both grids against
 // 94 of the staged deposit, 10 of them per-tile work.  Both grids of 1e8
@@ -1621,7 +1623,7 @@ paint_rot_kernel(PaintParams pp, const uint32_t *__restrict__ off, const uint4 *
 // have 32 distinct digits (and the half warps 16 distinct bank pairs each).
 // 1e6 particles at Ng = 128, both grids: 2.44 ms with 512-thread CTAs that
 // pulled the neighbours' particles and added with shared FP64 atomics, whose
-// compare-and-swap loops repeat the addition for a whole warp.
+// compare-and-swap loops repeat the addition for a whole warp; 0.78 so.
 constexpr int kF64Ext[3] = {8, 8, 16};
 constexpr int kF64BJ = (8 + 4) / 4, kF64BK = (16 + 4) / 4;  // j and k blocks of the box
 constexpr int kF64Blocks = (8 + 4) / 2 * kF64BJ * kF64BK;
